@@ -275,12 +275,14 @@ typedef enum {
     KBFV_TUNE_BCONV_THREADS = 4, /* 64, 128, 256 (default) or 512: CTA size of the base conversion
                                     Q -> R (the multiply's K2 and kbfv_bconv_*) */
     KBFV_TUNE_K5_THREADS = 5,    /* 64, 128 (default) or 256: CTA size of the multiply's
-                                    scale-and-round / R -> Q / digit-lift kernels (K5) */
-    KBFV_TUNE_K5_FUSED_PAIRS = 6, /* 0..128 (default 2): batches of at most this many pairs run K5
-                                    as one kernel, larger ones as two (fewer registers each) */
-    KBFV_TUNE_BCONV_CPT = 7,     /* 1 or 2 (default): coefficients per thread of the Q -> R base
-                                    conversion (2: 16-byte loads and stores, table reads shared by
-                                    two independent multiply-accumulate chains) */
+                                    scale-and-round / R -> Q and digit-lift kernels (K5) */
+    KBFV_TUNE_K5_FUSED_PAIRS = 6, /* 0..128 (default 2): batches of at most this many pairs run the
+                                    digit lift inside K5 (key switches with one digit of all
+                                    ciphertext primes), larger ones as a second kernel */
+    KBFV_TUNE_BCONV_CPT = 7,     /* 1 or 2 (default): coefficients per thread of the standalone base
+                                    conversions kbfv_bconv_* (2: 16-byte accesses and byte matrix
+                                    products on the tensor cores, as in the multiply; 1, and pointers
+                                    that are only 8-byte aligned: 64-bit multiply-accumulates) */
     KBFV_TUNE_FUSE_Q2R_PAIRS = 8, /* 0..128 (default 1): multiplies of at most this many pairs (per
                                     sub-batch) run the Q -> R base extension in the loader of the
                                     forward NTT over R: the inverse NTT over Q stores its outputs

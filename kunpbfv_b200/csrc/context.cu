@@ -1,6 +1,7 @@
 // libkbfv: context construction (parameter tables in one device pool), the
 // scratch arena, parameter sets, tuning knobs, the arithmetic-rate probe, the
 // noise budget and the wire format.
+#include "limb_mma.cuh"
 #include "pipeline.cuh"
 
 thread_local std::string g_last_error;
@@ -66,6 +67,51 @@ HostBconv make_bconv(const std::vector<uint64_t>& in, const std::vector<uint64_t
         for (size_t a = 0; a <= nin; a++) b.alpha[a * nout + j] = H::mulmod(a, bm, o);
     }
     return b;
+}
+
+// A byte matrix table (limb_mma.cuh): outputs j < nout mod mods[j], words w <
+// nwords with constants coef(j, w), and base(j) = B mod mods[j] of the quotient
+// term; ng column groups of 8 outputs, ks steps of 4 words, padding zero.
+template <class Coef, class Base>
+std::vector<uint8_t> mma_table(int ks, int ng, int nout, int nwords, const std::vector<uint64_t>& mods, Coef coef,
+                               Base base) {
+    std::vector<uint8_t> bytes(mma_table_bytes(ks, ng), 0);
+    MmaOut* out = (MmaOut*)bytes.data();
+    uint32_t* b = (uint32_t*)(bytes.data() + (size_t)ng * 8 * sizeof(MmaOut));
+    std::vector<uint64_t> c((size_t)nout * nwords * 8);  // (2^(8 byte) coef mod m) << sh
+    for (int j = 0; j < ng * 8; j++) {
+        // a padding output reduces zero modulo some 60-bit number
+        const uint64_t m = j < nout ? mods[j] : ((uint64_t)1 << 60) - 1;
+        const int sh = 60 - H::bit_count(m);
+        out[j].nm = 0 - (m << sh);
+        out[j].mu = (uint32_t)(((unsigned __int128)1 << 91) / (m << sh));
+        out[j].sh = (uint32_t)sh;
+        if (j >= nout) continue;
+        const uint64_t bm = base(j);
+        out[j].nb = (bm ? m - bm : 0) << sh;
+        for (int w = 0; w < nwords; w++) {
+            uint64_t v = coef(j, w) % m;
+            for (int byte = 0; byte < 8; byte++) {
+                c[((size_t)j * nwords + w) * 8 + byte] = v << sh;
+                v = H::mulmod(v, 256 % m, m);
+            }
+        }
+    }
+    for (int G = 0; G < ng; G++)
+        for (int s = 0; s < ks; s++)
+            for (int t = 0; t < 8; t++)
+                for (int lane = 0; lane < 32; lane++) {
+                    const int n = lane >> 2, j = (n >> 1) * 2 * ng + 2 * G + (n & 1), w = (lane & 3) * ks + s;
+                    if (j >= nout || w >= nwords) continue;
+                    const uint64_t* cw = &c[((size_t)j * nwords + w) * 8];
+                    for (int half = 0; half < 2; half++) {
+                        uint32_t f = 0;
+                        for (int byte = 0; byte < 4; byte++)
+                            f |= (uint32_t)((cw[4 * half + byte] >> (8 * t)) & 255) << (8 * byte);
+                        b[((((size_t)G * ks + s) * 4 + t / 2) * 32 + lane) * 4 + 2 * (t & 1) + half] = f;
+                    }
+                }
+    return bytes;
 }
 
 void gaussian_cdt(double sigma, int bound, std::vector<uint64_t>& table) {
@@ -317,6 +363,54 @@ void build_context(Context& c, const kbfv_params& prm) {
                     H::mulmod((uint64_t)v, dqm[(size_t)d * npq + m], c.mods[m]);
     size_t o_ks[11] = {blob.add(pmq), blob.add(pinv), blob.add(pinvs), blob.add(phi), blob.add(phis),
                        blob.add(phm), blob.add(dhi), blob.add(dhis), blob.add(dhm), blob.add(dqm), blob.add(dvq)};
+    // byte matrix tables of the base conversions
+    dc.mm_ks = mma_steps(c.mma_primes ? c.mma_primes : c.nq);
+    const int rgroups = mma_r_groups(dc.mm_ks);
+    const size_t o_mmq2r = blob.add(mma_table(
+        dc.mm_ks, rgroups, c.nr, c.nq, R, [&](int j, int w) { return q2r.hat[(size_t)j * c.nq + w]; },
+        [&](int j) { return q2r.alpha[(size_t)c.nr + j]; }));
+    const size_t o_mmsr = blob.add(mma_table(
+        dc.mm_ks, rgroups, c.nr, c.nq + 1, R,
+        [&](int j, int w) {
+            return w == c.nq ? r2q.hatinv[j] : H::mulmod(sr_c[(size_t)j * (c.nq + 1) + w], r2q.hatinv[j], R[j]);
+        },
+        [](int) { return (uint64_t)0; }));
+    const size_t o_mmr2q = blob.add(mma_table(
+        2 * rgroups, rgroups, c.nq, c.nr, Q, [&](int j, int w) { return r2q.hat[(size_t)j * c.nr + w]; },
+        [&](int j) { return r2q.alpha[(size_t)c.nq + j]; }));
+    size_t o_mmlift = 0;
+    {
+        const int ks = lift_steps(c.alpha);
+        int most = 0;
+        for (int d = 0; d < c.dnum; d++)
+            most = std::max(most, mma_groups(npq - std::max(0, std::min((d + 1) * c.alpha, c.nq) - d * c.alpha)));
+        dc.mm_lift_stride = mma_table_bytes(ks, most);
+        std::vector<uint8_t> all(dc.mm_lift_stride * c.dnum, 0);
+        for (int d = 0; d < c.dnum; d++) {
+            const int lo = d * c.alpha, n = std::max(0, std::min(lo + c.alpha, c.nq) - lo), nout = npq - n;
+            std::vector<uint64_t> om(nout);
+            for (int j = 0; j < nout; j++) om[j] = c.mods[j < lo ? j : j + n];
+            auto prime = [&](int j) { return (size_t)d * npq + (j < lo ? j : j + n); };
+            const std::vector<uint8_t> t = mma_table(
+                ks, mma_groups(nout), nout, n, om, [&](int j, int w) { return dhm[prime(j) * c.alpha + w]; },
+                [&](int j) { return dqm[prime(j)]; });
+            std::copy(t.begin(), t.end(), all.begin() + dc.mm_lift_stride * d);
+        }
+        o_mmlift = blob.add(all);
+    }
+    // K4 stores its R limbs times c_jj (R/r_j)^-1: the last inverse stage's constants take the factor
+    std::vector<tw_t> qr_fold((size_t)2 * (c.nq + c.nr));
+    for (int l = 0; l < c.nq + c.nr; l++) {
+        const int pi = l < c.nq ? l : dc.idx_r + (l - c.nq), j = l - c.nq;
+        const uint64_t q = c.mods[pi];
+        const uint64_t f = l < c.nq ? 1 : H::mulmod(sr_c[(size_t)j * (c.nq + 1) + c.nq], r2q.hatinv[j], q);
+        for (int k = 0; k < 2; k++) {
+            const uint64_t v = H::mulmod(twi[((size_t)pi << c.logn) + k].x, f, q);
+            qr_fold[2 * l + k].x = v;
+            qr_fold[2 * l + k].y = H::shoup(v, q);
+        }
+    }
+    const size_t o_qrf = blob.add(qr_fold);
     // T-base key switch constants (include/BasisConv.cuh:11-226; the reference's
     // precompute is in include/BFVcontext.cuh). Blocks lift by approximate CRT:
     // (B/b_j)^-1 mod b_j, B/b_j mod t_k and B mod t_k per block B.
@@ -420,6 +514,8 @@ void build_context(Context& c, const kbfv_params& prm) {
     dc.phatinv_ps = U(o_ks[4]); dc.phat_mod_q = U(o_ks[5]); dc.dig_hatinv = U(o_ks[6]);
     dc.dig_hatinvs = U(o_ks[7]); dc.dig_hat_mod = U(o_ks[8]); dc.dig_q_mod = U(o_ks[9]);
     dc.dig_vq_mod = U(o_ks[10]);
+    dc.mm_q2r = base + o_mmq2r; dc.mm_sr = base + o_mmsr; dc.mm_r2q = base + o_mmr2q; dc.mm_lift = base + o_mmlift;
+    dc.qr_fold = (const tw_t*)(base + o_qrf);
     dc.ms_qlinv = U(o_ms[0]); dc.ms_qlinvs = U(o_ms[1]); dc.ms_half_mod = U(o_ms[2]);
     dc.gauss_cdt = U(o_cdt);
     if (c.klss_ok) {

@@ -62,6 +62,14 @@ struct DevConsts {
     const uint64_t *p_mod_q, *pinv_q, *pinv_qs, *phatinv_p, *phatinv_ps, *phat_mod_q;
     const uint64_t *dig_hatinv, *dig_hatinvs, *dig_hat_mod, *dig_q_mod;
     const uint64_t* dig_vq_mod;  // [d][v = 0..alpha][npq]: v * Q_d mod p_m
+    // byte matrix tables of the base conversions (limb_mma.cuh), mm_ks steps:
+    // Q -> R, scale-and-round (times (R/r_j)^-1), R -> Q, and the digit lifts
+    // (mm_lift_stride bytes per digit)
+    const void *mm_q2r, *mm_sr, *mm_r2q, *mm_lift;
+    uint64_t mm_lift_stride;
+    const tw_t* qr_fold;  // [nqr][2]: the inverse NTT's last-stage constants over Q|R, those of an R prime
+                          // times its scale-and-round constant and (R/r_j)^-1
+    int mm_ks;
     int key_nq, key_npq;         // limb layout of the relinearisation key (top level's Q and Q|P counts)
     // modulus switch: q_last^-1 mod q_i (+ Shoup), floor(q_last / 2) mod q_i, for i < nq - 1
     const uint64_t *ms_qlinv, *ms_qlinvs, *ms_half_mod;
@@ -107,6 +115,9 @@ struct Context {
     DevConsts dc{};
     // host copies used by host-side diagnostics
     std::vector<uint64_t> h_q2r_hatinv;
+    // ciphertext primes that size the byte matrix tables (a level's: its top
+    // level's, so that one kernel serves a mixed batch); 0: this context's own
+    int mma_primes = 0;
 
     // scratch arena (grows; never shrinks while the context lives)
     void* scratch = nullptr;

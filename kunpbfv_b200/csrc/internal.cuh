@@ -244,9 +244,16 @@ static inline RowsIO rows_io(const DevConsts& dc, uint64_t* base, int p0, int pe
         else { MACRO(33); }                 \
     } while (0)
 
-// HPS base extension of `polys` polynomials (bconv_kernel), in and out strided
-void launch_bconv(const DevConsts& dc, const BconvTables& tb, const uint64_t* in, uint64_t* out, int polys,
-                  size_t in_stride, size_t out_stride, cudaStream_t st);
+// the same by the steps of the byte matrix products (DevConsts::mm_ks)
+#define DISPATCH_KS(ks, MACRO)          \
+    do {                                \
+        if ((ks) == 1) { MACRO(1); }    \
+        else if ((ks) == 2) { MACRO(2); } \
+        else if ((ks) == 4) { MACRO(4); } \
+        else if ((ks) == 6) { MACRO(6); } \
+        else { MACRO(9); }              \
+    } while (0)
+
 // context construction from a parameter set (tables in one device pool)
 void build_context(Context& c, const kbfv_params& prm);
 // pieces of a 60-bit residue in base 2^w

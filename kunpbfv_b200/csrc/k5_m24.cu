@@ -1,7 +1,9 @@
-// K5 kernels for contexts of at most 23 ciphertext primes (the MAXQ = 24 bucket)
+// K2, K5 and the fused K3 for contexts of 16 to 23 ciphertext primes
 #include "k5_kernels.cuh"
 
 template void q2r_ntt_launch_m<24>(const DevConsts&, const uint64_t*, uint64_t*, int, cudaStream_t);
-template void k5_launch_m<24>(const DevConsts&, int, const MulScratch&, uint64_t*, int, cudaStream_t);
-template void bconv_mixed_launch_m<24>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);
-template void k5_mixed_launch_m<24>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);
+template void k2_launch_m<6>(const DevConsts&, const uint64_t*, uint64_t*, int, cudaStream_t);
+template void bconv_mma_launch_m<6>(const DevConsts&, bool, const uint64_t*, uint64_t*, int, cudaStream_t);
+template void k5_launch_m<6>(const DevConsts&, int, const MulScratch&, uint64_t*, int, cudaStream_t);
+template void k2_mixed_launch_m<6>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);
+template void k5_mixed_launch_m<6>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);

@@ -14,20 +14,6 @@ namespace kbfv {
 // HPS base extension (BaseConverter::bConv_HPS, include/BasisConv_QR.cuh:191-207;
 // include/poly_arithmetic.cuh:1078-1178): centred lift of x mod B into O.
 // ===========================================================================
-// Per-coefficient kernels over a 2-D grid (x: chunks of `chunk` coefficients,
-// y: polynomials of `nrows` limbs, `poly_stride` words apart): threads
-// 0 .. nrows-1 ask L2 for their limb's chunk of the CTA `ahead` places later in
-// launch order (ahead = CTAs resident at once; 0: none), so that CTA's loads
-// hit L2 instead of waiting on HBM.
-__device__ __forceinline__ void prefetch_chunk_ahead(const uint64_t* in, size_t poly_stride, int nrows, int logn,
-                                                     int chunk, int ahead) {
-    if (ahead <= 0 || (int)threadIdx.x >= nrows) return;
-    const unsigned lin = blockIdx.y * gridDim.x + blockIdx.x + (unsigned)ahead;
-    if (lin >= gridDim.x * gridDim.y) return;
-    const unsigned bx = lin % gridDim.x, by = lin / gridDim.x;
-    l2_prefetch(in + by * poly_stride + ((size_t)threadIdx.x << logn) + (size_t)bx * chunk, (uint32_t)chunk * 8);
-}
-
 template <int MAXIN>
 __device__ __forceinline__ long long bconv_prep(uint64_t* y, const uint64_t* x, int nin,
                                                 const uint64_t* __restrict__ in_mods,
@@ -80,9 +66,8 @@ __host__ __device__ inline BconvTables r2q_tables(const DevConsts& c) {
 // one thread per coefficient; grid.y = polynomial
 template <int MAXIN>
 static __global__ void bconv_kernel(BconvTables tb, const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
-                             int logn, size_t in_stride, size_t out_stride, int ahead) {
+                             int logn, size_t in_stride, size_t out_stride) {
     extern __shared__ uint64_t sh_hat[];
-    prefetch_chunk_ahead(in, in_stride, tb.nin, logn, blockDim.x, ahead);
     for (int i = threadIdx.x; i < tb.nin * tb.nout; i += blockDim.x) sh_hat[i] = tb.hat[i];
     __syncthreads();
     const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,50 +81,6 @@ static __global__ void bconv_kernel(BconvTables tb, const uint64_t* __restrict__
     for (int j = 0; j < tb.nout; j++) {
         dst[((size_t)j << logn) + k] = bconv_out<MAXIN>(y, tb.nin, sh_hat + j * tb.nin, tb.alpha[v * tb.nout + j],
                                                         tb.out_mods[j], tb.out_mu_hi[j], tb.out_mu_lo[j]);
-    }
-}
-
-// Two coefficients per thread (k and k + 1: 16-byte loads and stores): the
-// table reads of each output prime (the hat row in shared memory, modulus,
-// Barrett constants) serve both, and the two multiply-accumulate chains are
-// independent. Per coefficient the arithmetic is bconv_kernel's.
-template <int MAXIN>
-static __global__ void bconv2_kernel(BconvTables tb, const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
-                                     int logn, size_t in_stride, size_t out_stride, int ahead) {
-    extern __shared__ uint64_t sh_hat[];
-    prefetch_chunk_ahead(in, in_stride, tb.nin, logn, 2 * blockDim.x, ahead);
-    for (int i = threadIdx.x; i < tb.nin * tb.nout; i += blockDim.x) sh_hat[i] = tb.hat[i];
-    __syncthreads();
-    const size_t k = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
-    const uint64_t* src = in + blockIdx.y * in_stride;
-    uint64_t* dst = out + blockIdx.y * out_stride;
-    uint64_t y0[MAXIN], y1[MAXIN];
-#pragma unroll
-    for (int i = 0; i < MAXIN; i++) {
-        if (i < tb.nin) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + ((size_t)i << logn) + k);
-            y0[i] = v.x;
-            y1[i] = v.y;
-        }
-    }
-    const long long v0 = bconv_prep<MAXIN>(y0, y0, tb.nin, tb.in_mods, tb.hatinv, tb.hatinvs, tb.binv);
-    const long long v1 = bconv_prep<MAXIN>(y1, y1, tb.nin, tb.in_mods, tb.hatinv, tb.hatinvs, tb.binv);
-    for (int j = 0; j < tb.nout; j++) {
-        const uint64_t* hr = sh_hat + j * tb.nin;
-        const uint64_t o = tb.out_mods[j], mh = tb.out_mu_hi[j], ml = tb.out_mu_lo[j];
-        u128 a0{0, 0}, a1{0, 0};
-#pragma unroll
-        for (int i = 0; i < MAXIN; i++) {
-            if (i < tb.nin) {
-                const uint64_t h = hr[i];
-                mac(a0, y0[i], h);
-                mac(a1, y1[i], h);
-            }
-        }
-        ulonglong2 r;
-        r.x = sub_mod(barrett128(a0, o, mh, ml), tb.alpha[v0 * tb.nout + j], o);
-        r.y = sub_mod(barrett128(a1, o, mh, ml), tb.alpha[v1 * tb.nout + j], o);
-        *reinterpret_cast<ulonglong2*>(dst + ((size_t)j << logn) + k) = r;
     }
 }
 

@@ -149,10 +149,10 @@ static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& p
     int n = 0;
     // K1: INTT over Q of [a1, b1, a2, b2]
     const StageRows r1 = stage_rows(G, [&](int g) { return 4 * G.nq[g]; }, &n);
-    ntt_inv(dc, MixedPairQRows{pb, G, r1}, MixedRows{m.sa, (size_t)4 * G.top_nq, G, r1, 0}, n, st);
+    ntt_inv(dc, MixedPairQRows{pb, G, r1}, MixedFoldRows{{m.sa, (size_t)4 * G.top_nq, G, r1, 0}}, n, st);
     // K2: Q -> R
-#define L_BM(M) bconv_mixed_launch_m<M>(G, dc.shape, count, m, st)
-    DISPATCH_MAXQ(G.top_nq + 1, L_BM);
+#define L_BM(K) k2_mixed_launch_m<K>(G, dc.shape, count, m, st)
+    DISPATCH_KS(dc.mm_ks, L_BM);
 #undef L_BM
     // K3: NTT over R in place, fully reduced
     const StageRows r3 = stage_rows(G, [&](int g) { return 4 * G.nr[g]; }, &n);
@@ -160,11 +160,12 @@ static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& p
     ntt_fwd<MixedRows, MixedRows, true>(dc, rrows, rrows, n, st);
     // K4: tensor fused into INTT over Q|R
     const StageRows r4 = stage_rows(G, [&](int g) { return 3 * G.nqr[g]; }, &n);
-    ntt_inv(dc, MixedTensorSrc{pb, m.sb, G, r4}, MixedRows{m.sc, (size_t)3 * G.top_nqr, G, r4, 3}, n, st);
+    ntt_inv(dc, MixedTensorSrc{pb, m.sb, G, r4}, MixedFoldRows{{m.sc, (size_t)3 * G.top_nqr, G, r4, 3}}, n, st);
     // K5: scale-and-round, R -> Q, digit lift
-#define L_KM(M) k5_mixed_launch_m<M>(G, dc.shape, count, m, st)
-    DISPATCH_MAXQ(G.top_nq + 1, L_KM);
+#define L_KM(K) k5_mixed_launch_m<K>(G, dc.shape, count, m, st)
+    DISPATCH_KS(dc.mm_ks, L_KM);
 #undef L_KM
+    lift_mixed_launch(G, dc, m.sd2, count, st);
     // K6a: NTT over Q|P of the digits in place, fully reduced
     const StageRows r6 = stage_rows(G, [&](int g) { return G.dnum[g] * G.npq[g]; }, &n);
     const MixedRows drows{m.sd2, (size_t)G.top_dnum * G.top_npq, G, r6, 2};
@@ -207,6 +208,7 @@ int kbfv_context_at_level(kbfv_context* ctx, uint32_t live_q, kbfv_context** out
             prm.p = c.mods.data() + c.nq;
             prm.digit_primes = (uint32_t)c.alpha;
             auto* h = new kbfv_context();
+            h->c.mma_primes = c.nq;  // mixed batches run every level's tables with one kernel
             try {
                 build_context(h->c, prm);
             } catch (...) {
@@ -441,12 +443,8 @@ int kbfv_apply_galois(kbfv_context* ctx, const uint64_t* d_gk, uint64_t galois_e
                                                                         m.sb + (size_t)i * lq, galois_elt, lq);
             check_launch("galois_b");
             // g(a) read through the permutation by the inverse NTT, then the hybrid key switch
-            ntt_inv(dc, GaloisASrc{in, galois_elt, dc.logn, dc.nq}, rows_io(dc, m.sa, 0, dc.nq), cnt * dc.nq, st);
-            dim3 grid((unsigned)(c.n / 128), (unsigned)cnt);
-#define L_MU(M) modup_kernel<M><<<grid, 128, 0, st>>>(dc, m.sa, m.sd2)
-            DISPATCH_MAXQ(dc.nq, L_MU);
-#undef L_MU
-            check_launch("modup");
+            ntt_inv(dc, GaloisASrc{in, galois_elt, dc.logn, dc.nq}, digit_rows(dc, m.sd2), cnt * dc.nq, st);
+            lift_launch(dc, m.sd2, cnt, st);
             ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sd2, 0, dc.npq), rows_io(dc, m.sd2, 0, dc.npq),
                                           cnt * dc.dnum * dc.npq, st);
             std::vector<uint64_t*> O(cnt);

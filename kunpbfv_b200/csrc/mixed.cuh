@@ -101,6 +101,17 @@ struct MixedRows {
     }
 };
 
+// MixedRows whose stored values carry a constant folded into the inverse
+// transform's last stage: K1's Q rows (kind 0, QHatRowsIO) and K4's Q|R rows
+// (kind 3, QRFoldRowsIO)
+struct MixedFoldRows : MixedRows {
+    __device__ __forceinline__ const tw_t* fold(int row) const {
+        const RowLoc L = locate(G, R, row);
+        const DevConsts* lv = G.lv[L.g];
+        return kind == 0 ? lv->q2r_fold + 2 * (int)G.dq[L.g].mod(L.local) : lv->qr_fold + 2 * (int)G.dqr[L.g].mod(L.local);
+    }
+};
+
 // K1 source: the Q limbs of [a1, b1, a2, b2] of each pair, in the pair's own
 // layout ([a | b], its level's live primes each)
 struct MixedPairQRows {
@@ -310,43 +321,9 @@ struct MixedOutCtKeyDst {
 };
 static inline MixedOutCtDst plain_of(const MixedOutCtKeyDst& d) { return MixedOutCtDst{d.pb, d.G, d.R}; }
 
-// K2 and K5 of a mixed batch (instantiated per MAXQ bucket in k5_m<MAXQ>.cu)
-template <int MAXQ>
-void bconv_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st);
-template <int MAXQ>
+// K2, K5 and the digit lift of a mixed batch (k5_kernels.cuh, lift.cu)
+template <int KS>
+void k2_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st);
+template <int KS>
 void k5_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st);
-
-// The level constants of item `item` copied into shared memory by the CTA (one
-// item per CTA row of the per-coefficient kernels), so that the kernels' reads
-// of them cannot alias their global stores.
-__device__ __forceinline__ void load_level_consts(DevConsts& dst, const DevConsts* src) {
-    static_assert(sizeof(DevConsts) % 8 == 0, "DevConsts copies as 8-byte words");
-    const uint64_t* s = reinterpret_cast<const uint64_t*>(src);
-    uint64_t* d = reinterpret_cast<uint64_t*>(&dst);
-    for (int i = threadIdx.x; i < (int)(sizeof(DevConsts) / 8); i += blockDim.x) d[i] = s[i];
-    __syncthreads();
-}
-
-// K2 over a mixed batch: Q -> R of [a1, b1, a2, b2] per item (grid.y = item x 4)
-template <int MAXIN>
-static __global__ void bconv_mixed_kernel(Groups G, const uint64_t* __restrict__ sa, uint64_t* __restrict__ sb) {
-    __shared__ DevConsts c;
-    extern __shared__ uint64_t sh_hat[];
-    const int item = blockIdx.y / 4, p = blockIdx.y % 4, g = G.group_of_item(item);
-    load_level_consts(c, G.lv[g]);
-    const BconvTables tb = q2r_tables(c);
-    for (int i = threadIdx.x; i < tb.nin * tb.nout; i += blockDim.x) sh_hat[i] = tb.hat[i];
-    __syncthreads();
-    const int logn = G.logn;
-    const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t* src = sa + (((size_t)item * 4 * G.top_nq + (size_t)p * tb.nin) << logn);
-    uint64_t* dst = sb + (((size_t)item * 4 * G.top_nr + (size_t)p * tb.nout) << logn);
-    uint64_t x[MAXIN], y[MAXIN];
-#pragma unroll
-    for (int i = 0; i < MAXIN; i++)
-        if (i < tb.nin) x[i] = src[((size_t)i << logn) + k];
-    const long long v = bconv_prep<MAXIN>(y, x, tb.nin, tb.in_mods, tb.hatinv, tb.hatinvs, tb.binv);
-    for (int j = 0; j < tb.nout; j++)
-        dst[((size_t)j << logn) + k] = bconv_out<MAXIN>(y, tb.nin, sh_hat + j * tb.nin, tb.alpha[v * tb.nout + j],
-                                                        tb.out_mods[j], tb.out_mu_hi[j], tb.out_mu_lo[j]);
-}
+void lift_mixed_launch(const Groups& G, const DevConsts& top, uint64_t* sd2, int count, cudaStream_t st);

@@ -24,30 +24,30 @@ void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int 
 }
 
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st) {
+    // K1: INTT over Q of [a1, b1, a2, b2], stored as y_i = [x_i (Q/q_i)^-1]_{q_i}
+    ntt_inv(dc, PairQRowsP{pb, dc.logn, dc.nq}, QHatRowsIO{m.sa, dc.logn, dc.nq, dc.q2r_fold}, count * 4 * dc.nq, st);
     if (count <= dc.shape.fuse_q2r_pairs) {
-        // K1 stores y_i = [x_i (Q/q_i)^-1]_{q_i}; K3's loader extends them to R
-        ntt_inv(dc, PairQRowsP{pb, dc.logn, dc.nq}, QHatRowsIO{m.sa, dc.logn, dc.nq, dc.q2r_fold},
-                count * 4 * dc.nq, st);
+        // K3's loader extends them to R
 #define L_Q2R(M) q2r_ntt_launch_m<M>(dc, m.sa, m.sb, count * 4, st)
         DISPATCH_MAXQ(dc.nq, L_Q2R);
 #undef L_Q2R
     } else {
-        // K1: INTT over Q of [a1, b1, a2, b2]
-        ntt_inv(dc, PairQRowsP{pb, dc.logn, dc.nq}, rows_io(dc, m.sa, 0, dc.nq), count * 4 * dc.nq, st);
         // K2: Q -> R (centred)
-        launch_bconv(dc, q2r_tables(dc), m.sa, m.sb, count * 4, (size_t)dc.nq << dc.logn, (size_t)dc.nr << dc.logn, st);
+#define L_K2(K) k2_launch_m<K>(dc, m.sa, m.sb, count * 4, st)
+        DISPATCH_KS(dc.mm_ks, L_K2);
+#undef L_K2
         // K3: NTT over R in place, fully reduced (the tensor's products use barrett_prod)
         ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sb, dc.idx_r, dc.nr), rows_io(dc, m.sb, dc.idx_r, dc.nr),
                                        count * 4 * dc.nr, st);
     }
     // K4: tensor (Q part from the NTT-form inputs, R part from K3) fused into INTT over Q|R
     TensorSrc ts{pb, m.sb, dc};
-    ntt_inv(dc, ts, QRRowsIO{m.sc, dc.logn, dc.nq, dc.nqr, dc.idx_r}, count * 3 * dc.nqr, st);
+    ntt_inv(dc, ts, QRFoldRowsIO{m.sc, dc.logn, dc.nq, dc.nqr, dc.idx_r, dc.qr_fold}, count * 3 * dc.nqr, st);
 }
 
 void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st) {
-#define L_K5(M) k5_launch_m<M>(dc, count, m, out0, mode, st)
-    DISPATCH_MAXQ(dc.nq + 1, L_K5);
+#define L_K5(K) k5_launch_m<K>(dc, count, m, out0, mode, st)
+    DISPATCH_KS(dc.mm_ks, L_K5);
 #undef L_K5
 }
 
@@ -116,13 +116,9 @@ int kbfv_relinearize(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_t* d
             MulScratch m = mul_scratch_layout(c, cnt, base);
             const uint64_t* tz = d_tensor + (size_t)off * 3 * lq;
             uint64_t* out = d_ct + (size_t)off * 2 * lq;
-            // INTT of a1*a2 into sa: rows (item, limb) read from the tensor's first poly
-            ntt_inv(dc, TensorA2{tz, dc.logn, dc.nq}, rows_io(dc, m.sa, 0, dc.nq), cnt * dc.nq, st);
-            dim3 grid((unsigned)(c.n / 128), (unsigned)cnt);
-#define L_MU(M) modup_kernel<M><<<grid, 128, 0, st>>>(dc, m.sa, m.sd2)
-            DISPATCH_MAXQ(dc.nq, L_MU);
-#undef L_MU
-            check_launch("modup");
+            // INTT of a1*a2 (rows (item, limb) of the tensor's first poly) into the digits' own limbs, then the lift
+            ntt_inv(dc, TensorA2{tz, dc.logn, dc.nq}, digit_rows(dc, m.sd2), cnt * dc.nq, st);
+            lift_launch(dc, m.sd2, cnt, st);
             ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sd2, 0, dc.npq), rows_io(dc, m.sd2, 0, dc.npq),
                                            cnt * dc.dnum * dc.npq, st);
             std::vector<uint64_t*> O(cnt);

@@ -50,23 +50,23 @@ static void ntt_rows(const Context& c, RowsIO io, int rows, bool fwd, cudaStream
     }
 }
 
-void launch_bconv(const DevConsts& dc, const BconvTables& tb, const uint64_t* in, uint64_t* out, int polys,
-                         size_t in_stride, size_t out_stride, cudaStream_t st) {
+// Standalone base conversions: the byte matrix product (two coefficients a
+// lane, 16-byte accesses), or one coefficient per thread where the caller's
+// pointers are only 8-byte aligned or the knob asks for it.
+static void launch_bconv(const DevConsts& dc, bool q2r, const uint64_t* in, uint64_t* out, int polys, cudaStream_t st) {
     if (polys <= 0) return;
-    const int threads = dc.shape.bconv_threads, cpt = dc.shape.bconv_cpt;
-    dim3 grid((unsigned)((1u << dc.logn) / (threads * cpt)), (unsigned)polys);
+    if (dc.shape.bconv_cpt == 2 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
+#define L_BM(K) bconv_mma_launch_m<K>(dc, q2r, in, out, polys, st)
+        DISPATCH_KS(dc.mm_ks, L_BM);
+#undef L_BM
+        return;
+    }
+    const BconvTables tb = q2r ? q2r_tables(dc) : r2q_tables(dc);
+    const int threads = dc.shape.bconv_threads;
+    dim3 grid((unsigned)((1u << dc.logn) / threads), (unsigned)polys);
     const size_t sh = (size_t)tb.nin * tb.nout * 8;
-#define L_BC(M)                                                                                            \
-    do {                                                                                                   \
-        static int res1[4] = {0, 0, 0, 0}, res2[4] = {0, 0, 0, 0};                                         \
-        if (cpt == 2) {                                                                                    \
-            const int a = dc.shape.l2_prefetch ? resident_ctas_at((const void*)bconv2_kernel<M>, threads, (int)sh, res2) : 0; \
-            bconv2_kernel<M><<<grid, threads, sh, st>>>(tb, in, out, dc.logn, in_stride, out_stride, a);   \
-        } else {                                                                                           \
-            const int a = dc.shape.l2_prefetch ? resident_ctas_at((const void*)bconv_kernel<M>, threads, (int)sh, res1) : 0; \
-            bconv_kernel<M><<<grid, threads, sh, st>>>(tb, in, out, dc.logn, in_stride, out_stride, a);    \
-        }                                                                                                  \
-    } while (0)
+#define L_BC(M)                                                                                                 \
+    bconv_kernel<M><<<grid, threads, sh, st>>>(tb, in, out, dc.logn, (size_t)tb.nin << dc.logn, (size_t)tb.nout << dc.logn)
     DISPATCH_MAXQ(tb.nin, L_BC);
 #undef L_BC
     check_launch("bconv");
@@ -109,16 +109,14 @@ int kbfv_ntt_inv(kbfv_context* ctx, uint64_t* d_rows, uint32_t rows, uint32_t pr
 int kbfv_bconv_q_to_r(kbfv_context* ctx, const uint64_t* d_in, uint64_t* d_out, uint32_t polys, kbfv_stream stream) {
     return guarded([&] {
         Context& c = CX(ctx);
-        launch_bconv(c.dc, q2r_tables(c.dc), d_in, d_out, (int)polys, (size_t)c.nq << c.logn,
-                     (size_t)c.nr << c.logn, S(stream));
+        launch_bconv(c.dc, true, d_in, d_out, (int)polys, S(stream));
     });
 }
 
 int kbfv_bconv_r_to_q(kbfv_context* ctx, const uint64_t* d_in, uint64_t* d_out, uint32_t polys, kbfv_stream stream) {
     return guarded([&] {
         Context& c = CX(ctx);
-        launch_bconv(c.dc, r2q_tables(c.dc), d_in, d_out, (int)polys, (size_t)c.nr << c.logn,
-                     (size_t)c.nq << c.logn, S(stream));
+        launch_bconv(c.dc, false, d_in, d_out, (int)polys, S(stream));
     });
 }
 

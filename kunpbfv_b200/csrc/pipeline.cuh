@@ -19,8 +19,7 @@ struct PairQRowsP {
     __device__ __forceinline__ void prefetch(int row, int off, int n) const { bind(row).prefetch(off, n); }
 };
 
-// K1 store target when the Q -> R base extension runs inside K3: rows over Q
-// (RowsIO layout) holding y_i = [x_i (Q/q_i)^-1]_{q_i}, the scale folded into
+// K1 store target: rows over Q (RowsIO layout) holding the base extension's words y_i = [x_i (Q/q_i)^-1]_{q_i}, the scale folded into
 // the inverse transform's last-stage constants
 struct QHatRowsIO {
     uint64_t* base;
@@ -32,14 +31,17 @@ struct QHatRowsIO {
 };
 
 // rows of consecutive Q|R polynomials; limb l of Q|R uses prime l (Q) or idx_r + l - nq (R)
-struct QRRowsIO {
+// (K4's store target: an R limb times its scale-and-round constant and (R/r_j)^-1, see qr_fold)
+struct QRFoldRowsIO {
     uint64_t* base;
     int logn, nq, nqr, idx_r;
+    const tw_t* fold_base;  // DevConsts::qr_fold
     __device__ __forceinline__ int prime(int row) const {
         const int l = row % nqr;
         return l < nq ? l : idx_r + (l - nq);
     }
     __device__ __forceinline__ PtrRow bind(int row) const { return PtrRow{base + ((size_t)row << logn)}; }
+    __device__ __forceinline__ const tw_t* fold(int row) const { return fold_base + 2 * (row % nqr); }
 };
 
 // K4 source: tensor product of the pair at limb l of Q|R, one of three outputs
@@ -347,17 +349,39 @@ struct DecSrc {
 };
 
 
+// an inverse transform's rows (item, limb of Q) stored at the digits' own limbs:
+// [item][dnum][Q|P], limb i in digit i / alpha
+struct DigitRowsIO {
+    uint64_t* sd2;
+    int logn, nq, npq, dnum, alpha;
+    __device__ __forceinline__ int prime(int row) const { return row % nq; }
+    __device__ __forceinline__ PtrRow bind(int row) const {
+        const int item = row / nq, l = row % nq;
+        return PtrRow{sd2 + ((((size_t)item * dnum + l / alpha) * npq + l) << logn)};
+    }
+};
+static inline DigitRowsIO digit_rows(const DevConsts& dc, uint64_t* sd2) {
+    return DigitRowsIO{sd2, dc.logn, dc.nq, dc.npq, dc.dnum, dc.alpha};
+}
+
 // INTT over Q of the four input polynomials, Q -> R, NTT over R, fused tensor +
 // INTT over Q|R: steps shared by kbfv_mul and the fused multiply-relinearise.
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st);
-// K5: scale-and-round, R -> Q and (mode 1) the key-switch digit lift
-template <int MAXQ>
+// K2 and K5 (k5_kernels.cuh), by the steps of the byte matrix products
+template <int KS>
+void k2_launch_m(const DevConsts& dc, const uint64_t* y, uint64_t* out, int polys, cudaStream_t st);
+template <int KS>
+void bconv_mma_launch_m(const DevConsts& dc, bool q2r, const uint64_t* in, uint64_t* out, int polys, cudaStream_t st);
+template <int KS>
 void k5_launch_m(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st);
 // K3 with the Q -> R base extension in its loader: `polys` polynomials of y
 // rows over Q (QHatRowsIO layout) -> NTT-form R limbs, fully reduced
 template <int MAXQ>
 void q2r_ntt_launch_m(const DevConsts& dc, const uint64_t* y, uint64_t* out, int polys, cudaStream_t st);
+// K5: scale-and-round, R -> Q and (mode 1) the key-switch digit lift
 void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st);
+// the key-switch lift of the digits' own limbs in sd2 ([item][dnum][npq]) into every other prime of Q|P (lift.cu)
+void lift_launch(const DevConsts& dc, uint64_t* sd2, int count, cudaStream_t st);
 // key-switch tail: key product, mod down and add, written to the outputs of pb
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
              const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st);
