@@ -70,12 +70,14 @@ HostBconv make_bconv(const std::vector<uint64_t>& in, const std::vector<uint64_t
 }
 
 // A byte matrix table (limb_mma.cuh): outputs j < nout mod mods[j], words w <
-// nwords with constants coef(j, w), and base(j) = B mod mods[j] of the quotient
-// term; ng column groups of 8 outputs, ks steps of 4 words, padding zero.
-template <class Coef, class Base>
-std::vector<uint8_t> mma_table(int ks, int ng, int nout, int nwords, const std::vector<uint64_t>& mods, Coef coef,
-                               Base base) {
-    std::vector<uint8_t> bytes(mma_table_bytes(ks, ng), 0);
+// nwords with constants coef(j, w); ng column groups of 8 outputs, ks steps of 4
+// words, padding zero. `extra`: the last word is in a step of its own (step ks,
+// lane 0 of the quad).
+template <class Coef>
+std::vector<uint8_t> mma_table(int ks, bool extra, int ng, int nout, int nwords, const std::vector<uint64_t>& mods,
+                               Coef coef) {
+    const int steps = ks + (extra ? 1 : 0);
+    std::vector<uint8_t> bytes(mma_table_bytes(steps, ng), 0);
     MmaOut* out = (MmaOut*)bytes.data();
     uint32_t* b = (uint32_t*)(bytes.data() + (size_t)ng * 8 * sizeof(MmaOut));
     std::vector<uint64_t> c((size_t)nout * nwords * 8);  // (2^(8 byte) coef mod m) << sh
@@ -87,8 +89,6 @@ std::vector<uint8_t> mma_table(int ks, int ng, int nout, int nwords, const std::
         out[j].mu = (uint32_t)(((unsigned __int128)1 << 91) / (m << sh));
         out[j].sh = (uint32_t)sh;
         if (j >= nout) continue;
-        const uint64_t bm = base(j);
-        out[j].nb = (bm ? m - bm : 0) << sh;
         for (int w = 0; w < nwords; w++) {
             uint64_t v = coef(j, w) % m;
             for (int byte = 0; byte < 8; byte++) {
@@ -98,17 +98,18 @@ std::vector<uint8_t> mma_table(int ks, int ng, int nout, int nwords, const std::
         }
     }
     for (int G = 0; G < ng; G++)
-        for (int s = 0; s < ks; s++)
+        for (int s = 0; s < steps; s++)
             for (int t = 0; t < 8; t++)
                 for (int lane = 0; lane < 32; lane++) {
-                    const int n = lane >> 2, j = (n >> 1) * 2 * ng + 2 * G + (n & 1), w = (lane & 3) * ks + s;
-                    if (j >= nout || w >= nwords) continue;
+                    const int n = lane >> 2, j = (n >> 1) * 2 * ng + 2 * G + (n & 1);
+                    const int w = s < ks ? (lane & 3) * ks + s : (lane & 3) == 0 ? nwords - 1 : nwords;
+                    if (j >= nout || w >= (s < ks && extra ? nwords - 1 : nwords)) continue;
                     const uint64_t* cw = &c[((size_t)j * nwords + w) * 8];
                     for (int half = 0; half < 2; half++) {
                         uint32_t f = 0;
                         for (int byte = 0; byte < 4; byte++)
                             f |= (uint32_t)((cw[4 * half + byte] >> (8 * t)) & 255) << (8 * byte);
-                        b[((((size_t)G * ks + s) * 4 + t / 2) * 32 + lane) * 4 + 2 * (t & 1) + half] = f;
+                        b[((((size_t)G * steps + s) * 4 + t / 2) * 32 + lane) * 4 + 2 * (t & 1) + half] = f;
                     }
                 }
     return bytes;
@@ -366,18 +367,20 @@ void build_context(Context& c, const kbfv_params& prm) {
     // byte matrix tables of the base conversions
     dc.mm_ks = mma_steps(c.mma_primes ? c.mma_primes : c.nq);
     const int rgroups = mma_r_groups(dc.mm_ks);
-    const size_t o_mmq2r = blob.add(mma_table(
-        dc.mm_ks, rgroups, c.nr, c.nq, R, [&](int j, int w) { return q2r.hat[(size_t)j * c.nq + w]; },
-        [&](int j) { return q2r.alpha[(size_t)c.nr + j]; }));
-    const size_t o_mmsr = blob.add(mma_table(
-        dc.mm_ks, rgroups, c.nr, c.nq + 1, R,
-        [&](int j, int w) {
-            return w == c.nq ? r2q.hatinv[j] : H::mulmod(sr_c[(size_t)j * (c.nq + 1) + w], r2q.hatinv[j], R[j]);
-        },
-        [](int) { return (uint64_t)0; }));
-    const size_t o_mmr2q = blob.add(mma_table(
-        2 * rgroups, rgroups, c.nq, c.nr, Q, [&](int j, int w) { return r2q.hat[(size_t)j * c.nr + w]; },
-        [&](int j) { return r2q.alpha[(size_t)c.nq + j]; }));
+    dc.mm_shift = 0;
+    for (uint64_t m : Q) dc.mm_shift |= H::bit_count(m) < 60;
+    for (uint64_t m : R) dc.mm_shift |= H::bit_count(m) < 60;
+    // -v mod m as the constant of the quotient word
+    auto neg = [](uint64_t v, uint64_t m) { return v ? m - v : 0; };
+    const size_t o_mmq2r = blob.add(mma_table(dc.mm_ks, false, rgroups, c.nr, c.nq + 1, R, [&](int j, int w) {
+        return w == c.nq ? neg(q2r.alpha[(size_t)c.nr + j], R[j]) : q2r.hat[(size_t)j * c.nq + w];
+    }));
+    const size_t o_mmsr = blob.add(mma_table(dc.mm_ks, false, rgroups, c.nr, c.nq + 1, R, [&](int j, int w) {
+        return w == c.nq ? r2q.hatinv[j] : H::mulmod(sr_c[(size_t)j * (c.nq + 1) + w], r2q.hatinv[j], R[j]);
+    }));
+    const size_t o_mmr2q = blob.add(mma_table(2 * rgroups, true, rgroups, c.nq, c.nr + 1, Q, [&](int j, int w) {
+        return w == c.nr ? neg(r2q.alpha[(size_t)c.nq + j], Q[j]) : r2q.hat[(size_t)j * c.nr + w];
+    }));
     size_t o_mmlift = 0;
     {
         const int ks = lift_steps(c.alpha);
@@ -391,9 +394,9 @@ void build_context(Context& c, const kbfv_params& prm) {
             std::vector<uint64_t> om(nout);
             for (int j = 0; j < nout; j++) om[j] = c.mods[j < lo ? j : j + n];
             auto prime = [&](int j) { return (size_t)d * npq + (j < lo ? j : j + n); };
-            const std::vector<uint8_t> t = mma_table(
-                ks, mma_groups(nout), nout, n, om, [&](int j, int w) { return dhm[prime(j) * c.alpha + w]; },
-                [&](int j) { return dqm[prime(j)]; });
+            const std::vector<uint8_t> t = mma_table(ks, false, mma_groups(nout), nout, n + 1, om, [&](int j, int w) {
+                return w == n ? neg(dqm[prime(j)], om[j]) : dhm[prime(j) * c.alpha + w];
+            });
             std::copy(t.begin(), t.end(), all.begin() + dc.mm_lift_stride * d);
         }
         o_mmlift = blob.add(all);

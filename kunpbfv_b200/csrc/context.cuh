@@ -70,6 +70,7 @@ struct DevConsts {
     const tw_t* qr_fold;  // [nqr][2]: the inverse NTT's last-stage constants over Q|R, those of an R prime
                           // times its scale-and-round constant and (R/r_j)^-1
     int mm_ks;
+    int mm_shift;  // 1: some prime of Q or R has fewer than 60 bits
     int key_nq, key_npq;         // limb layout of the relinearisation key (top level's Q and Q|P counts)
     // modulus switch: q_last^-1 mod q_i (+ Shoup), floor(q_last / 2) mod q_i, for i < nq - 1
     const uint64_t *ms_qlinv, *ms_qlinvs, *ms_half_mod;

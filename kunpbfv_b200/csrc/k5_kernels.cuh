@@ -6,9 +6,9 @@
 // translation unit (k5_m<MAXQ>.cu) so that the unrolled variants compile in
 // parallel.
 //
-// A warp takes 16 coefficients of one polynomial per iteration: lane
-// (g = lane / 4, c = lane % 4) coefficients 2g and 2g + 1, the words and outputs
-// of limb_mma.cuh. A CTA's iterations take consecutive runs of coefficients.
+// A warp takes MT tiles of 16 coefficients of one polynomial per iteration: lane
+// (g = lane / 4, c = lane % 4) coefficients 2g and 2g + 1 of each, the words and
+// outputs of limb_mma.cuh. A CTA's iterations take consecutive runs of coefficients.
 //
 // The figures at the kernels are of N = 16384, 7 + 1 primes, 32 pairs (2^21
 // coefficients in K2, 1.5 x 2^20 in K5), one launch under ncu, against the same
@@ -18,29 +18,100 @@
 #include "mixed.cuh"
 #include "q2r_ntt.cuh"
 
-// iterations of a CTA of `threads` threads (threads / 2 coefficients each): as
-// few as leave four waves of CTAs, so that small launches cover the SMs and
-// large ones load the constants of a lane (held in registers across the
-// iterations) rarely
-static inline int mma_iters(size_t polys, int logn, int threads, int resident) {
-    const size_t per = ((size_t)1 << logn) / (threads / 2);  // iterations that one polynomial takes (a power of two)
+// Tiles per iteration: two share one load of the constants as long as their
+// words and sums fit the registers of at least 16 warps per SM.
+constexpr int mma_tiles(int ks) { return ks <= 2 ? 2 : 1; }
+// Tables of up to 20 KiB are copied to shared memory by each CTA; larger ones
+// (16 primes and more) are read through L1.
+constexpr bool mma_staged(int ks) { return ks <= 5; }
+constexpr int mma_stage_bytes(int ks, int ng) { return mma_staged(ks) ? (int)mma_table_bytes(ks, ng) : 0; }
+
+// iterations of a CTA that takes `each` coefficients at a time: as few as leave
+// four waves of CTAs, so that small launches cover the SMs and large ones load
+// a lane's constants rarely
+static inline int mma_iters(size_t polys, int logn, int each, int resident) {
+    const size_t per = ((size_t)1 << logn) / each;  // iterations that one polynomial takes (a power of two)
     size_t it = 1;
     while (it < per && it < 16 && polys * per / (2 * it) >= (size_t)4 * resident) it *= 2;
     return (int)it;
 }
+// CTAs of a launch
+static inline unsigned mma_blocks(size_t polys, int logn, int each, int iters) {
+    return (unsigned)(polys * (((size_t)1 << logn) / ((size_t)each * iters)));
+}
 
-// the CTA's polynomial and first coefficient, the warp's place in an iteration
+// the CTA's polynomial and first coefficient, the lane's place in it; a warp's
+// second tile follows its first by 16 coefficients
 struct MmaPlace {
     int poly;
     size_t k;    // coefficient of the lane's row 0 in iteration 0
-    int lane, c;
+    size_t warp; // first coefficient of the warp in iteration 0
+    int own;     // the warp's coefficient whose floating-point sum the lane takes (16 MT lanes; the others repeat)
+    int at;      // the lane's row 0 among the warp's coefficients
+    int lane, c, each;
 };
+template <int MT>
 __device__ __forceinline__ MmaPlace mma_place(int logn, int iters) {
-    const unsigned per = (1u << logn) / ((blockDim.x / 2) * iters);
-    const int lane = threadIdx.x & 31;
-    return MmaPlace{(int)(blockIdx.x / per),
-                    (size_t)(blockIdx.x % per) * (blockDim.x / 2) * iters + (threadIdx.x >> 5) * 16 + 2 * (lane >> 2),
-                    lane, lane & 3};
+    const int lane = threadIdx.x & 31, each = blockDim.x / 2 * MT;
+    const unsigned per = (1u << logn) / (each * iters);
+    const size_t warp = (size_t)(blockIdx.x % per) * each * iters + (threadIdx.x >> 5) * 16 * MT;
+    return MmaPlace{(int)(blockIdx.x / per), warp + 2 * (lane >> 2), warp, lane % (16 * MT), 2 * (lane >> 2), lane,
+                    lane & 3, each};
+}
+// the 32-bit value that each coefficient's owner holds as the word of the last step (lane 0 of the quad)
+template <int KS, int MT>
+__device__ __forceinline__ void put_extra(uint64_t (&w)[MT][2][KS], uint32_t own, const MmaPlace& pl) {
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint32_t v = __shfl_sync(0xffffffffu, own, 16 * m + pl.at + r);
+            w[m][r][KS - 1] = pl.c == 0 ? v : 0;
+        }
+    }
+}
+// the value that each coefficient's owner holds (T: 32 or 64 bits) as word `word` of the lanes that have it
+template <int KS, int MT, class T>
+__device__ __forceinline__ void put_word(uint64_t (&w)[MT][2][KS], T own, int word, const MmaPlace& pl) {
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const T v = __shfl_sync(0xffffffffu, own, 16 * m + pl.at + r);
+#pragma unroll
+            for (int s = 0; s < KS; s++)
+                if (pl.c * KS + s == word) w[m][r][s] = v;
+        }
+    }
+}
+// The words of a warp's coefficients, copied to a buffer of its own in shared
+// memory (rows of 16 MT coefficients, padded by 16 bytes) while it computes the
+// iteration before: the copies are asynchronous, the lanes that need a word as a
+// fragment and the lane that needs it in a floating-point sum read the same copy
+// (loaded to registers when needed, K2 took 88 us at 51% issue, waiting on loads).
+template <int MT>
+constexpr int kRow = 16 * MT + 2;
+template <int MT, int MAXW>
+__device__ __forceinline__ void copy_words(uint64_t* buf, const uint64_t* src, int n, int logn, int lane) {
+    constexpr int PER = 8 * MT;  // 16-byte pieces of a word's row
+    const int piece = lane % PER, w0 = lane / PER;
+    const uint64_t* s = src + ((size_t)w0 << logn) + 2 * piece;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(buf + w0 * kRow<MT> + 2 * piece);
+#pragma unroll
+    for (int t = 0; t < MAXW; t += 32 / PER)
+        if (t + w0 < n)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + t * kRow<MT> * 8), "l"(s + ((size_t)t << logn))
+                         : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all copies but the newest group have arrived, for the whole warp
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ ulonglong2 load2(const uint64_t* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ void store2(uint64_t* p, uint64_t x, uint64_t y) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x, y);
 }
 
 // ---------------------------------------------------------------------------
@@ -89,71 +160,108 @@ struct MixedExtJob {
     }
 };
 
-// K2, 32 pairs: 179 us with 64-bit multiply-accumulates -> 87 us here
-template <int KS, int NG, bool PREP, class Job>
-static __global__ void ext_mma_kernel(Job job, int logn, int iters) {
-    const MmaPlace pl = mma_place(logn, iters);
+// K2, 32 pairs: 179 us with 64-bit multiply-accumulates -> 61 us here (252 MB
+// moved: 38 us at the copy rate; issue-bound at 480 instructions per 32 coefficients)
+// EXTRA: the quotient word has a step of its own (R -> Q), else it is word nin.
+template <int KS, int NG, bool EXTRA, bool PREP, bool SH, class Job>
+static __global__ void __maxnreg__(KS <= 4 && !PREP ? 80 : 128) ext_mma_kernel(Job job, int logn, int iters) {
+    constexpr int MT = mma_tiles(KS), STEPS = KS + (EXTRA ? 1 : 0), BUF = 4 * KS * kRow<MT>;
+    extern __shared__ uint4 mma_sh[];
+    const MmaPlace pl = mma_place<MT>(logn, iters);
     const ExtPoly e = job.bind(pl.poly);
+    double* binv = (double*)(mma_sh + mma_stage_bytes(STEPS, NG) / 16);
+    uint64_t* buf = (uint64_t*)(binv + 4 * KS) + (threadIdx.x >> 5) * 2 * BUF;
+    const uint64_t* in = e.in + pl.warp;
+    copy_words<MT, 4 * KS>(buf, in, e.nin, logn, pl.lane);
+    copy_commit();
+    if (mma_staged(STEPS)) mma_stage(mma_sh, e.tab, STEPS);
+    if ((int)threadIdx.x < e.nin) binv[threadIdx.x] = __ldg(e.binv + threadIdx.x);
+    __syncthreads();
+    const MmaTab tab = mma_staged(STEPS) ? mma_tab(mma_sh, NG) : e.tab;
     const int first = pl.c * KS;
-    double f[KS];
-    MmaOut o[2 * NG];
+    uint64_t* out = e.out + ((size_t)(pl.c * 2 * NG) << logn) + pl.k;
+    for (int it = 0; it < iters; it++, out += pl.each) {
+        const uint64_t* cur = buf + (it & 1) * BUF;
+        in += pl.each;
+        if (it + 1 < iters) copy_words<MT, 4 * KS>(buf + (~it & 1) * BUF, in, e.nin, logn, pl.lane);
+        copy_commit();
+        copy_wait();
+        double frac = 0.0;
 #pragma unroll
-    for (int s = 0; s < KS; s++) f[s] = first + s < e.nin ? e.binv[first + s] : 0.0;
-#pragma unroll
-    for (int i = 0; i < 2 * NG; i++)
-        if (NG <= 2) o[i] = mma_out(e.tab.out + pl.c * 2 * NG + i);
-    size_t k = pl.k;
-    for (int it = 0; it < iters; it++, k += blockDim.x / 2) {
-        uint64_t w[2][KS];
-        double x0[KS], x1[KS];
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-            ulonglong2 v = make_ulonglong2(0, 0);
-            if (first + s < e.nin) {
-                v = *reinterpret_cast<const ulonglong2*>(e.in + ((size_t)(first + s) << logn) + k);
-                if (PREP) {
-                    const uint64_t h = e.hatinv[first + s], hs = e.hatinvs[first + s], m = e.mods[first + s];
-                    v.x = shoup(v.x, h, hs, m);
-                    v.y = shoup(v.y, h, hs, m);
-                }
+        for (int i = 0; i < 4 * KS; i++) {
+            if (i < e.nin) {
+                uint64_t y = cur[i * kRow<MT> + pl.own];
+                if (PREP) y = shoup(y, __ldg(e.hatinv + i), __ldg(e.hatinvs + i), __ldg(e.mods + i));
+                frac = __fma_rn(__ull2double_rn(y), binv[i], frac);
             }
-            w[0][s] = v.x;
-            w[1][s] = v.y;
         }
+        uint64_t w[MT][2][STEPS];
 #pragma unroll
-        for (int s = 0; s < KS; s++) {
-            x0[s] = u64_to_double(w[0][s]);
-            x1[s] = u64_to_double(w[1][s]);
+        for (int s = 0; s < STEPS; s++) {
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                ulonglong2 x = make_ulonglong2(0, 0);
+                if (s < KS && first + s < e.nin) x = load2(cur + (first + s) * kRow<MT> + 16 * m + pl.at);
+                w[m][0][s] = x.x;
+                w[m][1][s] = x.y;
+            }
         }
-        const uint32_t v0 = (uint32_t)llround(quad_fma_sum<KS>(x0, f, 0.0, first, e.nin));
-        const uint32_t v1 = (uint32_t)llround(quad_fma_sum<KS>(x1, f, 0.0, first, e.nin));
+        if (PREP) {
+#pragma unroll
+            for (int s = 0; s < KS; s++) {
+                if (first + s >= e.nin) continue;
+                const uint64_t h = __ldg(e.hatinv + first + s), hs = __ldg(e.hatinvs + first + s),
+                               q = __ldg(e.mods + first + s);
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int r = 0; r < 2; r++) w[m][r][s] = shoup(w[m][r][s], h, hs, q);
+            }
+        }
+        if (EXTRA) put_extra<STEPS>(w, round_half_up(frac), pl);
+        else put_word<STEPS>(w, round_half_up(frac), e.nin, pl);
 #pragma unroll
         for (int G = 0; G < NG; G++) {
-            int S[8][4];
-            mma_digits<KS>(S, w, e.tab, G, pl.lane);
+            uint32_t D[MT][4][4];
+            mma_digits<STEPS, MT>(D, w, tab, G, pl.lane);
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int j = pl.c * 2 * NG + 2 * G + i;
-                if (j >= e.nout) continue;
-                const MmaOut oo = NG <= 2 ? o[2 * G + i] : mma_out(e.tab.out + j);
-                ulonglong2 r;
-                r.x = mma_value<false>(S, i, v0, 0, oo);
-                r.y = mma_value<false>(S, 2 + i, v1, 0, oo);
-                *reinterpret_cast<ulonglong2*>(e.out + ((size_t)j << logn) + k) = r;
+                const MmaOut o = mma_out(tab.out + j);
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    const uint64_t r0 = mma_value<false, SH>(D[m], i, 0, o);
+                    const uint64_t r1 = mma_value<false, SH>(D[m], 2 + i, 0, o);
+                    if (j < e.nout) store2(out + ((size_t)(2 * G + i) << logn) + 16 * m, r0, r1);
+                }
             }
         }
+        __syncwarp();  // the buffer is read; the next iteration's copies overwrite it
     }
 }
 
-template <int KS, int NG, bool PREP, class Job>
-static void ext_mma_launch(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
-    if (polys <= 0) return;
+template <int KS, int NG, bool EXTRA, bool PREP, bool SH, class Job>
+static void ext_mma_launch_sh(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
     static int res[4] = {0, 0, 0, 0};
-    const int iters = mma_iters(polys, logn, threads,
-                                resident_ctas_at((const void*)ext_mma_kernel<KS, NG, PREP, Job>, threads, 0, res));
-    const size_t per = ((size_t)1 << logn) / ((size_t)(threads / 2) * iters);
-    ext_mma_kernel<KS, NG, PREP, Job><<<(unsigned)(polys * per), threads, 0, st>>>(job, logn, iters);
+    const int smem = mma_stage_bytes(KS + (EXTRA ? 1 : 0), NG) + 4 * KS * 8 +
+                     threads / 32 * 2 * 4 * KS * kRow<mma_tiles(KS)> * 8;
+    static int allowed = 48 << 10;  // dynamic shared memory of a launch without an attribute
+    if (smem > allowed) {
+        KB_CHECK_CUDA(cudaFuncSetAttribute(ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        allowed = smem;
+    }
+    const int each = threads / 2 * mma_tiles(KS);
+    const int iters = mma_iters(polys, logn, each,
+                                resident_ctas_at((const void*)ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, threads, smem, res));
+    ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job><<<mma_blocks(polys, logn, each, iters), threads, smem, st>>>(job, logn, iters);
     check_launch("base_extension");
+}
+template <int KS, int NG, bool EXTRA, bool PREP, class Job>
+static void ext_mma_launch(const Job& job, bool shifted, int polys, int logn, int threads, cudaStream_t st) {
+    if (polys <= 0) return;
+    if (shifted) ext_mma_launch_sh<KS, NG, EXTRA, PREP, true>(job, polys, logn, threads, st);
+    else ext_mma_launch_sh<KS, NG, EXTRA, PREP, false>(job, polys, logn, threads, st);
 }
 
 // K2: y rows over Q (QHatRowsIO layout) -> R limbs of `polys` polynomials
@@ -165,7 +273,7 @@ void k2_launch_m(const DevConsts& dc, const uint64_t* y, uint64_t* out, int poly
     job.p.binv = dc.q2r_inv;
     job.p.nin = dc.nq;
     job.p.nout = dc.nr;
-    ext_mma_launch<KS, NG, false>(job, polys, dc.logn, dc.shape.bconv_threads, st);
+    ext_mma_launch<KS, NG, false, false>(job, dc.mm_shift, polys, dc.logn, dc.shape.bconv_threads, st);
 }
 // the standalone conversions, from residues
 template <int KS>
@@ -180,8 +288,8 @@ void bconv_mma_launch_m(const DevConsts& dc, bool q2r, const uint64_t* in, uint6
     job.p.hatinv = tb.hatinv;
     job.p.hatinvs = tb.hatinvs;
     job.p.mods = tb.in_mods;
-    if (q2r) ext_mma_launch<KS, NG, true>(job, polys, dc.logn, dc.shape.bconv_threads, st);
-    else ext_mma_launch<2 * NG, NG, true>(job, polys, dc.logn, dc.shape.bconv_threads, st);
+    if (q2r) ext_mma_launch<KS, NG, false, true>(job, dc.mm_shift, polys, dc.logn, dc.shape.bconv_threads, st);
+    else ext_mma_launch<2 * NG, NG, true, true>(job, dc.mm_shift, polys, dc.logn, dc.shape.bconv_threads, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -198,19 +306,15 @@ struct LiftDigit {
     int lo, n, nout;
     const uint64_t *mods, *hatinv, *hatinvs;  // of the digit's first prime
 };
-// word i of the digit and its term of the quotient estimate, for the lane's two coefficients
-__device__ __forceinline__ void lift_word(const LiftDigit& d, int i, ulonglong2 v, uint64_t& w0, uint64_t& w1, float& x0,
-                                          float& x1) {
-    const uint64_t h = d.hatinv[i], hs = d.hatinvs[i], q = d.mods[i];
-    w0 = shoup(v.x, h, hs, q);
-    w1 = shoup(v.y, h, hs, q);
-    const float fq = __ull2float_rn(q);
-    x0 = __fdiv_rn(__ull2float_rn(w0), fq);
-    x1 = __fdiv_rn(__ull2float_rn(w1), fq);
+// word i of the digit and its term of the quotient estimate
+__device__ __forceinline__ void lift_word(const LiftDigit& d, int i, uint64_t x, uint64_t& w, float& t) {
+    const uint64_t q = d.mods[i];
+    w = shoup(x, d.hatinv[i], d.hatinvs[i], q);
+    t = __fdiv_rn(__ull2float_rn(w), __ull2float_rn(q));
 }
 // the quotient estimate of one coefficient: the quad's float terms added in index order
 template <int KS>
-__device__ __forceinline__ int lift_quotient(const float (&x)[KS], int first, int n, int alpha) {
+__device__ __forceinline__ uint32_t lift_quotient(const float (&x)[KS], int first, int n, int alpha) {
     float acc = 0.f;
 #pragma unroll
     for (int hop = 0; hop < 4; hop++) {
@@ -219,29 +323,25 @@ __device__ __forceinline__ int lift_quotient(const float (&x)[KS], int first, in
             if (first + s < n) acc = __fadd_rn(acc, x[s]);
         if (hop < 3) acc = __shfl_up_sync(0xffffffffu, acc, 1, 4);
     }
-    return min(__float2int_rz(__shfl_sync(0xffffffffu, acc, 3, 4)), alpha);
+    return (uint32_t)min(__float2int_rz(__shfl_sync(0xffffffffu, acc, 3, 4)), alpha);
 }
-
 // the digit's outputs over the primes outside it, stored at d.rows
-template <int KS>
-__device__ __forceinline__ void lift_outputs(const uint64_t (&w)[2][KS], const float (&x0)[KS], const float (&x1)[KS],
-                                             const LiftDigit& d, int logn, int alpha, int first, size_t k,
+template <int KS, int MT>
+__device__ __forceinline__ void lift_outputs(const uint64_t (&w)[MT][2][KS], const LiftDigit& d, const MmaTab& tab, int logn, size_t k,
                                              const MmaPlace& pl) {
-    const uint32_t v0 = (uint32_t)lift_quotient<KS>(x0, first, d.n, alpha);
-    const uint32_t v1 = (uint32_t)lift_quotient<KS>(x1, first, d.n, alpha);
-    const int ng = d.tab.ng;
+    const int ng = tab.ng;
     for (int G = 0; G < ng; G++) {
-        int S[8][4];
-        mma_digits<KS>(S, w, d.tab, G, pl.lane);
+        uint32_t D[MT][4][4];
+        mma_digits<KS, MT>(D, w, tab, G, pl.lane);
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int j = pl.c * 2 * ng + 2 * G + i;
             if (j >= d.nout) continue;
-            const MmaOut o = mma_out(d.tab.out + j);
-            ulonglong2 r;
-            r.x = mma_value<false>(S, i, v0, 0, o);
-            r.y = mma_value<false>(S, 2 + i, v1, 0, o);
-            *reinterpret_cast<ulonglong2*>(d.rows + ((size_t)(j < d.lo ? j : j + d.n) << logn) + k) = r;
+            const MmaOut o = mma_out(tab.out + j);
+            uint64_t* row = d.rows + ((size_t)(j < d.lo ? j : j + d.n) << logn);
+#pragma unroll
+            for (int m = 0; m < MT; m++)
+                store2(row + k + 16 * m, mma_value<false, true>(D[m], i, 0, o), mma_value<false, true>(D[m], 2 + i, 0, o));
         }
     }
 }
@@ -342,118 +442,169 @@ struct MixedK5Job {
     }
 };
 
-// K5, 32 pairs: 163 + 168 us (two kernels of 64-bit multiply-accumulates) -> 117 us here, the lift (lift.cuh) 31 us
+// K5, 32 pairs: 163 + 168 us (two kernels of 64-bit multiply-accumulates) -> 97 us here, the lift (lift.cuh) 26 us
 // FUSED: the digit lift too, where one digit holds all of Q and the R -> Q
 // product's outputs are the lift's words.
-template <int KS, int NG, bool FUSED, class Job>
-static __global__ void k5_mma_kernel(Job job, int logn, int iters) {
-    constexpr int K2 = 2 * NG;  // words a lane holds of the second product
-    const MmaPlace pl = mma_place(logn, iters);
+template <int KS, int NG, bool FUSED, bool SH, class Job>
+static __global__ void __launch_bounds__(256, KS <= 4 ? 3 : 1) k5_mma_kernel(Job job, int logn, int iters) {
+    constexpr int K2 = 2 * NG, MT = mma_tiles(KS);  // K2: words a lane holds of the second product
+    extern __shared__ uint4 mma_sh[];
+    const MmaPlace pl = mma_place<MT>(logn, iters);
     const K5Poly p = job.bind(pl.poly);
+    uint4* sh2 = mma_sh + mma_stage_bytes(KS, NG) / 16;
+    // two buffers of the nq + nr input words; the product's nr words go where its input's were
+    constexpr int BUF = 4 * (KS + K2) * kRow<MT>, Y0 = 4 * KS * kRow<MT>;
+    double* fr = (double*)(sh2 + mma_stage_bytes(K2 + 1, NG) / 16);  // factors of the two floating-point sums
+    uint64_t* buf = (uint64_t*)(fr + 4 * (KS + K2)) + (threadIdx.x >> 5) * 2 * BUF;
+    if (mma_staged(KS)) mma_stage(mma_sh, p.sr, KS);
+    if (mma_staged(K2 + 1)) mma_stage(sh2, p.r2q, K2 + 1);
+    for (int i = threadIdx.x; i < p.nq + p.nr; i += blockDim.x)
+        fr[i < p.nq ? i : 4 * KS + i - p.nq] = __ldg(i < p.nq ? p.sr_frac + i : p.r2q_inv + (i - p.nq));
     const int first = pl.c * KS, first2 = pl.c * K2;
-    double f[KS], f2[K2];
-#pragma unroll
-    for (int s = 0; s < KS; s++) f[s] = first + s < p.nq ? p.sr_frac[first + s] : 0.0;
-#pragma unroll
-    for (int s = 0; s < K2; s++) f2[s] = first2 + s < p.nr ? p.r2q_inv[first2 + s] : 0.0;
+    const uint64_t* in = p.src + pl.warp;
+    auto copy_in = [&](uint64_t* to) {
+        copy_words<MT, 4 * KS>(to, in, p.nq, logn, pl.lane);
+        copy_words<MT, 4 * K2>(to + Y0, in + ((size_t)p.nq << logn), p.nr, logn, pl.lane);
+    };
+    copy_in(buf);
+    copy_commit();
+    __syncthreads();
+    const MmaTab sr = mma_staged(KS) ? mma_tab(mma_sh, NG) : p.sr;
+    const MmaTab r2q = mma_staged(K2 + 1) ? mma_tab(sh2, NG) : p.r2q;
     size_t k = pl.k;
-    for (int it = 0; it < iters; it++, k += blockDim.x / 2) {
-        uint64_t y[2][K2];
+    for (int it = 0; it < iters; it++, k += pl.each) {
+        uint64_t* cur = buf + (it & 1) * BUF;
+        in += pl.each;
+        if (it + 1 < iters) copy_in(buf + (~it & 1) * BUF);
+        copy_commit();
+        copy_wait();
+        uint64_t y[MT][2][K2 + 1];
         {
-            uint64_t w[2][KS];
-            double x0[KS], x1[KS];
+            uint64_t w[MT][2][KS];
 #pragma unroll
             for (int s = 0; s < KS; s++) {
-                ulonglong2 v = make_ulonglong2(0, 0);
-                if (first + s < p.nq) v = *reinterpret_cast<const ulonglong2*>(p.src + ((size_t)(first + s) << logn) + k);
-                w[0][s] = v.x;
-                w[1][s] = v.y;
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    ulonglong2 x = make_ulonglong2(0, 0);
+                    if (first + s < p.nq) x = load2(cur + (first + s) * kRow<MT> + 16 * m + pl.at);
+                    w[m][0][s] = x.x;
+                    w[m][1][s] = x.y;
+                }
             }
 #pragma unroll
             for (int s = 0; s < K2; s++) {
-                ulonglong2 v = make_ulonglong2(0, 0);
-                if (first2 + s < p.nr)
-                    v = *reinterpret_cast<const ulonglong2*>(p.src + ((size_t)(p.nq + first2 + s) << logn) + k);
-                y[0][s] = v.x;
-                y[1][s] = v.y;
-            }
 #pragma unroll
-            for (int s = 0; s < KS; s++) {
-                x0[s] = u64_to_double(w[0][s]);
-                x1[s] = u64_to_double(w[1][s]);
-            }
-            const uint64_t a0 = __double2ull_rz(quad_fma_sum<KS>(x0, f, 0.5, first, p.nq));
-            const uint64_t a1 = __double2ull_rz(quad_fma_sum<KS>(x1, f, 0.5, first, p.nq));
-#pragma unroll
-            for (int s = 0; s < KS; s++) {
-                if (first + s == p.nq) {
-                    w[0][s] = a0;
-                    w[1][s] = a1;
+                for (int m = 0; m < MT; m++) {
+                    ulonglong2 x = make_ulonglong2(0, 0);
+                    if (first2 + s < p.nr) x = load2(cur + Y0 + (first2 + s) * kRow<MT> + 16 * m + pl.at);
+                    y[m][0][s] = x.x;
+                    y[m][1][s] = x.y;
                 }
             }
+            double nu = 0.5;
+#pragma unroll
+            for (int i = 0; i < 4 * KS; i++)
+                if (i < p.nq) nu = __fma_rn(__ull2double_rn(cur[i * kRow<MT> + pl.own]), fr[i], nu);
+            put_word<KS>(w, (uint64_t)__double2ull_rz(nu), p.nq, pl);
 #pragma unroll
             for (int G = 0; G < NG; G++) {
-                int S[8][4];
-                mma_digits<KS>(S, w, p.sr, G, pl.lane);
+                uint32_t D[MT][4][4];
+                mma_digits<KS, MT>(D, w, sr, G, pl.lane);
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    const MmaOut o = mma_out(p.sr.out + first2 + 2 * G + i);
-                    y[0][2 * G + i] = mma_value<true>(S, i, 0, y[0][2 * G + i], o);
-                    y[1][2 * G + i] = mma_value<true>(S, 2 + i, 0, y[1][2 * G + i], o);
+                    const MmaOut o = mma_out(sr.out + first2 + 2 * G + i);
+#pragma unroll
+                    for (int m = 0; m < MT; m++) {
+#pragma unroll
+                        for (int r = 0; r < 2; r++)
+                            y[m][r][2 * G + i] =
+                                mma_value<true, SH>(D[m], 2 * r + i, y[m][r][2 * G + i], o);
+                    }
                 }
             }
         }
-        double x0[K2], x1[K2];
+        // the words of a coefficient to the lane that sums them (each lane overwrites what it read itself)
 #pragma unroll
-        for (int s = 0; s < K2; s++) {
-            x0[s] = u64_to_double(y[0][s]);
-            x1[s] = u64_to_double(y[1][s]);
-        }
-        const uint32_t v0 = (uint32_t)llround(quad_fma_sum<K2>(x0, f2, 0.0, first2, p.nr));
-        const uint32_t v1 = (uint32_t)llround(quad_fma_sum<K2>(x1, f2, 0.0, first2, p.nr));
-        ulonglong2 x[FUSED ? K2 : 1];
+        for (int s = 0; s < K2; s++)
+#pragma unroll
+            for (int m = 0; m < MT; m++)
+                store2(cur + Y0 + (first2 + s) * kRow<MT> + 16 * m + pl.at, y[m][0][s], y[m][1][s]);
+        __syncwarp();
+        double frac = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4 * K2; i++)
+            if (i < p.nr) frac = __fma_rn(__ull2double_rn(cur[Y0 + i * kRow<MT> + pl.own]), fr[4 * KS + i], frac);
+        __syncwarp();  // the buffer is read; the next iteration's copies overwrite it
+        put_extra<K2 + 1>(y, round_half_up(frac), pl);
+        uint64_t x[FUSED ? MT : 1][2][FUSED ? K2 : 1];
 #pragma unroll
         for (int G = 0; G < NG; G++) {
-            int S[8][4];
-            mma_digits<K2>(S, y, p.r2q, G, pl.lane);
+            uint32_t D[MT][4][4];
+            mma_digits<K2 + 1, MT>(D, y, r2q, G, pl.lane);
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int j = first2 + 2 * G + i;
-                if (FUSED) x[2 * G + i] = make_ulonglong2(0, 0);
-                if (j >= p.nq) continue;
-                const MmaOut o = mma_out(p.r2q.out + j);
-                ulonglong2 r;
-                r.x = mma_value<false>(S, i, v0, 0, o);
-                r.y = mma_value<false>(S, 2 + i, v1, 0, o);
-                *reinterpret_cast<ulonglong2*>(p.dst + ((size_t)(j + j / p.alpha * p.digit) << logn) + k) = r;
-                if (FUSED) x[2 * G + i] = r;
+                const MmaOut o = mma_out(r2q.out + j);
+                uint64_t* row = p.dst + ((size_t)(p.digit ? j + j / p.alpha * p.digit : j) << logn);
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    const uint64_t r0 = mma_value<false, SH>(D[m], i, 0, o);
+                    const uint64_t r1 = mma_value<false, SH>(D[m], 2 + i, 0, o);
+                    if (j < p.nq) store2(row + k + 16 * m, r0, r1);
+                    if (FUSED) {
+                        x[FUSED ? m : 0][0][FUSED ? 2 * G + i : 0] = r0;
+                        x[FUSED ? m : 0][1][FUSED ? 2 * G + i : 0] = r1;
+                    }
+                }
             }
         }
         if constexpr (FUSED) {
             LiftDigit d;
             if (job.lift(pl.poly, p, d)) {  // the whole CTA's polynomial
-                uint64_t w[2][K2];
-                float t0[K2], t1[K2];
 #pragma unroll
-                for (int s = 0; s < K2; s++) {
-                    w[0][s] = w[1][s] = 0;
-                    t0[s] = t1[s] = 0.f;
-                    if (first2 + s < d.n) lift_word(d, first2 + s, x[s], w[0][s], w[1][s], t0[s], t1[s]);
+                for (int m = 0; m < MT; m++) {
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        float t[K2];
+#pragma unroll
+                        for (int s = 0; s < K2; s++) {
+                            t[s] = 0.f;
+                            if (first2 + s < d.n) lift_word(d, first2 + s, x[m][r][s], x[m][r][s], t[s]);
+                            else x[m][r][s] = 0;
+                        }
+                        const uint32_t v = lift_quotient<K2>(t, first2, d.n, p.alpha);
+#pragma unroll
+                        for (int s = 0; s < K2; s++)
+                            if (first2 + s == d.n) x[m][r][s] = v;
+                    }
                 }
-                lift_outputs<K2>(w, t0, t1, d, logn, p.alpha, first2, k, pl);
+                lift_outputs<K2, MT>(x, d, d.tab, logn, k, pl);
             }
         }
     }
 }
 
-template <int KS, int NG, bool FUSED, class Job>
-static void k5_mma_launch(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
+template <int KS, int NG, bool FUSED, bool SH, class Job>
+static void k5_mma_launch_sh(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
     static int res[4] = {0, 0, 0, 0};
-    const int iters = mma_iters(polys, logn, threads,
-                                resident_ctas_at((const void*)k5_mma_kernel<KS, NG, FUSED, Job>, threads, 0, res));
-    const size_t per = ((size_t)1 << logn) / ((size_t)(threads / 2) * iters);
-    k5_mma_kernel<KS, NG, FUSED, Job><<<(unsigned)(polys * per), threads, 0, st>>>(job, logn, iters);
+    const int smem = mma_stage_bytes(KS, NG) + mma_stage_bytes(2 * NG + 1, NG) + 4 * (KS + 2 * NG) * 8 +
+                     threads / 32 * 2 * 4 * (KS + 2 * NG) * kRow<mma_tiles(KS)> * 8;
+    const int each = threads / 2 * mma_tiles(KS);
+    static int allowed = 48 << 10;  // dynamic shared memory of a launch without an attribute
+    if (smem > allowed) {
+        KB_CHECK_CUDA(cudaFuncSetAttribute(k5_mma_kernel<KS, NG, FUSED, SH, Job>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        allowed = smem;
+    }
+    const int iters = mma_iters(polys, logn, each,
+                                resident_ctas_at((const void*)k5_mma_kernel<KS, NG, FUSED, SH, Job>, threads, smem, res));
+    k5_mma_kernel<KS, NG, FUSED, SH, Job><<<mma_blocks(polys, logn, each, iters), threads, smem, st>>>(job, logn, iters);
     check_launch("k5");
+}
+template <int KS, int NG, bool FUSED, class Job>
+static void k5_mma_launch(const Job& job, bool shifted, int polys, int logn, int threads, cudaStream_t st) {
+    if (shifted) k5_mma_launch_sh<KS, NG, FUSED, true>(job, polys, logn, threads, st);
+    else k5_mma_launch_sh<KS, NG, FUSED, false>(job, polys, logn, threads, st);
 }
 template <int KS>
 void k5_launch_m(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st) {
@@ -462,19 +613,19 @@ void k5_launch_m(const DevConsts& dc, int count, const MulScratch& m, uint64_t* 
     // small batches: one launch less on the per-call path; larger ones run the
     // lift, a third of K5's polynomials, as a kernel of fewer registers
     const bool fused = mode == 1 && dc.dnum == 1 && lift_steps(dc.alpha) == 2 * NG && count <= dc.shape.k5_fused_pairs;
-    if (fused) k5_mma_launch<KS, NG, true>(job, count * 3, dc.logn, dc.shape.k5_threads, st);
-    else k5_mma_launch<KS, NG, false>(job, count * 3, dc.logn, dc.shape.k5_threads, st);
+    if (fused) k5_mma_launch<KS, NG, true>(job, dc.mm_shift, count * 3, dc.logn, dc.shape.k5_threads, st);
+    else k5_mma_launch<KS, NG, false>(job, dc.mm_shift, count * 3, dc.logn, dc.shape.k5_threads, st);
     if (mode == 1 && !fused) lift_launch(dc, m.sd2, count, st);
 }
 
 // K2 and K5 of a mixed batch (KS of the top level's prime count, which its levels' tables share)
 template <int KS>
-void k2_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st) {
+void k2_mixed_launch_m(const Groups& G, const LaunchShape& sh, bool shifted, int count, const MulScratch& m, cudaStream_t st) {
     constexpr int NG = mma_r_groups(KS);
-    ext_mma_launch<KS, NG, false>(MixedExtJob<NG>{G, m.sa, m.sb}, count * 4, G.logn, sh.bconv_threads, st);
+    ext_mma_launch<KS, NG, false, false>(MixedExtJob<NG>{G, m.sa, m.sb}, shifted, count * 4, G.logn, sh.bconv_threads, st);
 }
 template <int KS>
-void k5_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st) {
+void k5_mixed_launch_m(const Groups& G, const LaunchShape& sh, bool shifted, int count, const MulScratch& m, cudaStream_t st) {
     constexpr int NG = mma_r_groups(KS);
-    k5_mma_launch<KS, NG, false>(MixedK5Job<NG>{G, m.sc, m.sd, m.sd2}, count * 3, G.logn, sh.k5_threads, st);
+    k5_mma_launch<KS, NG, false>(MixedK5Job<NG>{G, m.sc, m.sd, m.sd2}, shifted, count * 3, G.logn, sh.k5_threads, st);
 }

@@ -5,5 +5,5 @@ template void q2r_ntt_launch_m<33>(const DevConsts&, const uint64_t*, uint64_t*,
 template void k2_launch_m<9>(const DevConsts&, const uint64_t*, uint64_t*, int, cudaStream_t);
 template void bconv_mma_launch_m<9>(const DevConsts&, bool, const uint64_t*, uint64_t*, int, cudaStream_t);
 template void k5_launch_m<9>(const DevConsts&, int, const MulScratch&, uint64_t*, int, cudaStream_t);
-template void k2_mixed_launch_m<9>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);
-template void k5_mixed_launch_m<9>(const Groups&, const LaunchShape&, int, const MulScratch&, cudaStream_t);
+template void k2_mixed_launch_m<9>(const Groups&, const LaunchShape&, bool, int, const MulScratch&, cudaStream_t);
+template void k5_mixed_launch_m<9>(const Groups&, const LaunchShape&, bool, int, const MulScratch&, cudaStream_t);

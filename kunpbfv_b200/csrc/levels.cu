@@ -113,6 +113,8 @@ static void add_group(kbfv_context* top_h, Context& top, Groups& G, int lvl, int
     const int g = G.ng++;
     G.first[g] = first;
     G.lv[g] = level_consts(top_h, top, lvl);
+    const DevConsts& ldc = lvl == top.nq ? top.dc : ((kbfv_context*)top.levels[lvl])->c.dc;
+    G.lift_table = std::max(G.lift_table, ldc.mm_lift_stride);
     G.nq[g] = lvl;
     G.nr[g] = lvl + 1;
     G.npq[g] = lvl + top.np;
@@ -151,7 +153,7 @@ static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& p
     const StageRows r1 = stage_rows(G, [&](int g) { return 4 * G.nq[g]; }, &n);
     ntt_inv(dc, MixedPairQRows{pb, G, r1}, MixedFoldRows{{m.sa, (size_t)4 * G.top_nq, G, r1, 0}}, n, st);
     // K2: Q -> R
-#define L_BM(K) k2_mixed_launch_m<K>(G, dc.shape, count, m, st)
+#define L_BM(K) k2_mixed_launch_m<K>(G, dc.shape, dc.mm_shift, count, m, st)
     DISPATCH_KS(dc.mm_ks, L_BM);
 #undef L_BM
     // K3: NTT over R in place, fully reduced
@@ -162,7 +164,7 @@ static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& p
     const StageRows r4 = stage_rows(G, [&](int g) { return 3 * G.nqr[g]; }, &n);
     ntt_inv(dc, MixedTensorSrc{pb, m.sb, G, r4}, MixedFoldRows{{m.sc, (size_t)3 * G.top_nqr, G, r4, 3}}, n, st);
     // K5: scale-and-round, R -> Q, digit lift
-#define L_KM(K) k5_mixed_launch_m<K>(G, dc.shape, count, m, st)
+#define L_KM(K) k5_mixed_launch_m<K>(G, dc.shape, dc.mm_shift, count, m, st)
     DISPATCH_KS(dc.mm_ks, L_KM);
 #undef L_KM
     lift_mixed_launch(G, dc, m.sd2, count, st);

@@ -42,45 +42,71 @@ struct MixedLiftJob {
 };
 
 template <int KS, class Job>
-static __global__ void lift_mma_kernel(Job job, int logn, int alpha, int iters) {
-    const MmaPlace pl = mma_place(logn, iters);
+static __global__ void __launch_bounds__(256) lift_mma_kernel(Job job, int logn, int alpha, int iters, int stage) {
+    constexpr int MT = mma_tiles(KS);
+    const MmaPlace pl = mma_place<MT>(logn, iters);
+    extern __shared__ uint4 mma_sh[];
     LiftDigit d;
-    if (!job.bind(pl.poly, d)) return;
+    if (!job.bind(pl.poly, d)) return;  // the whole CTA
+    if (stage) {
+        mma_stage(mma_sh, d.tab, KS);
+        __syncthreads();
+    }
     const int first = pl.c * KS;
     size_t k = pl.k;
-    for (int it = 0; it < iters; it++, k += blockDim.x / 2) {
-        uint64_t w[2][KS];
-        float x0[KS], x1[KS];
+    for (int it = 0; it < iters; it++, k += pl.each) {
+        uint64_t w[MT][2][KS];
+        float t[MT][2][KS];
 #pragma unroll
         for (int s = 0; s < KS; s++) {
-            w[0][s] = w[1][s] = 0;
-            x0[s] = x1[s] = 0.f;
-            if (first + s < d.n) {
-                const ulonglong2 v =
-                    *reinterpret_cast<const ulonglong2*>(d.rows + ((size_t)(d.lo + first + s) << logn) + k);
-                lift_word(d, first + s, v, w[0][s], w[1][s], x0[s], x1[s]);
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                w[m][0][s] = w[m][1][s] = 0;
+                t[m][0][s] = t[m][1][s] = 0.f;
+                if (first + s < d.n) {
+                    const ulonglong2 x = load2(d.rows + ((size_t)(d.lo + first + s) << logn) + k + 16 * m);
+                    w[m][0][s] = x.x;
+                    w[m][1][s] = x.y;
+                }
             }
         }
-        lift_outputs<KS>(w, x0, x1, d, logn, alpha, first, k, pl);
+#pragma unroll
+        for (int s = 0; s < KS; s++)
+            if (first + s < d.n)
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+#pragma unroll
+                    for (int r = 0; r < 2; r++) lift_word(d, first + s, w[m][r][s], w[m][r][s], t[m][r][s]);
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const uint32_t v = lift_quotient<KS>(t[m][r], first, d.n, alpha);
+#pragma unroll
+                for (int s = 0; s < KS; s++)
+                    if (first + s == d.n) w[m][r][s] = v;
+            }
+        if (stage) lift_outputs<KS, MT>(w, d, mma_tab(mma_sh, d.tab.ng), logn, k, pl);
+        else lift_outputs<KS, MT>(w, d, d.tab, logn, k, pl);
     }
 }
 
 template <int KS, class Job>
-static void lift_mma_launch(const Job& job, int rows, int logn, int alpha, int threads, cudaStream_t st) {
-    static int res[4] = {0, 0, 0, 0};
+static void lift_mma_launch(const Job& job, size_t table, int rows, int logn, int alpha, int threads, cudaStream_t st) {
+    const int each = threads / 2 * mma_tiles(KS);
+    const int smem = table <= 16 << 10 ? (int)table : 0;  // larger tables are read through L1
     const int iters =
-        mma_iters(rows, logn, threads, resident_ctas_at((const void*)lift_mma_kernel<KS, Job>, threads, 0, res));
-    const size_t per = ((size_t)1 << logn) / ((size_t)(threads / 2) * iters);
-    lift_mma_kernel<KS, Job><<<(unsigned)(rows * per), threads, 0, st>>>(job, logn, alpha, iters);
+        mma_iters(rows, logn, each, resident_ctas((const void*)lift_mma_kernel<KS, Job>, threads, smem));
+    lift_mma_kernel<KS, Job><<<mma_blocks(rows, logn, each, iters), threads, smem, st>>>(job, logn, alpha, iters, smem != 0);
     check_launch("digit_lift");
 }
 template <class Job>
-static void lift_launch_any(const Job& job, int rows, int logn, int alpha, int threads, cudaStream_t st) {
+static void lift_launch_any(const Job& job, size_t table, int rows, int logn, int alpha, int threads, cudaStream_t st) {
     switch (lift_steps(alpha)) {
-        case 1: lift_mma_launch<1>(job, rows, logn, alpha, threads, st); break;
-        case 2: lift_mma_launch<2>(job, rows, logn, alpha, threads, st); break;
-        case 4: lift_mma_launch<4>(job, rows, logn, alpha, threads, st); break;
-        case 6: lift_mma_launch<6>(job, rows, logn, alpha, threads, st); break;
-        default: lift_mma_launch<10>(job, rows, logn, alpha, threads, st); break;
+        case 1: lift_mma_launch<1>(job, table, rows, logn, alpha, threads, st); break;
+        case 2: lift_mma_launch<2>(job, table, rows, logn, alpha, threads, st); break;
+        case 4: lift_mma_launch<4>(job, table, rows, logn, alpha, threads, st); break;
+        case 6: lift_mma_launch<6>(job, table, rows, logn, alpha, threads, st); break;
+        default: lift_mma_launch<10>(job, table, rows, logn, alpha, threads, st); break;
     }
 }

@@ -39,6 +39,7 @@ struct Groups {
     int logn, np;
     int top_nq, top_nr, top_npq, top_nqr, top_dnum;  // scratch layout per item (top level's)
     int key_nq, key_npq;                      // limb layout of the top-level key
+    uint64_t lift_table;                      // bytes of the largest digit-lift table of these levels
     __device__ __forceinline__ int group_of_item(int item) const {
         int g = 0;
         while (g + 1 < ng && item >= first[g + 1]) g++;
@@ -323,7 +324,9 @@ static inline MixedOutCtDst plain_of(const MixedOutCtKeyDst& d) { return MixedOu
 
 // K2, K5 and the digit lift of a mixed batch (k5_kernels.cuh, lift.cu)
 template <int KS>
-void k2_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st);
+void k2_mixed_launch_m(const Groups& G, const LaunchShape& sh, bool shifted, int count, const MulScratch& m,
+                       cudaStream_t st);
 template <int KS>
-void k5_mixed_launch_m(const Groups& G, const LaunchShape& sh, int count, const MulScratch& m, cudaStream_t st);
+void k5_mixed_launch_m(const Groups& G, const LaunchShape& sh, bool shifted, int count, const MulScratch& m,
+                       cudaStream_t st);
 void lift_mixed_launch(const Groups& G, const DevConsts& top, uint64_t* sd2, int count, cudaStream_t st);
