@@ -105,6 +105,12 @@ __device__ __forceinline__ uint64_t barrett_prod(u128 x, uint64_t q, uint64_t mu
     r = csub(r, q << 1);
     return csub(r, q);
 }
+// the same without the conditional subtractions: [0, 4q), for consumers that take lazy values
+__device__ __forceinline__ uint64_t barrett_prod_lazy(u128 x, uint64_t q, uint64_t mu) {
+    const int s = 62 - __clzll(q);
+    const uint64_t t = (x.lo >> s) | (x.hi << (64 - s));
+    return x.lo - __umul64hi(t, mu) * q;
+}
 __device__ __forceinline__ uint64_t mul_mod_prod(uint64_t a, uint64_t b, uint64_t q, uint64_t mu) {
     return barrett_prod(mul_wide(a, b), q, mu);
 }

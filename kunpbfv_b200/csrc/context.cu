@@ -414,6 +414,22 @@ void build_context(Context& c, const kbfv_params& prm) {
         }
     }
     const size_t o_qrf = blob.add(qr_fold);
+    // the key-switch tail's mod down: K6b stores rb_k = [x_k (P/p_k)^-1]_{p_k}, K7 multiplies by -(P/p_k) P^-1
+    std::vector<tw_t> p_fold((size_t)2 * c.np), md_c((size_t)c.nq * c.np);
+    for (int k = 0; k < c.np; k++) {
+        const uint64_t q = P[k];
+        for (int i = 0; i < 2; i++) {
+            const uint64_t v = H::mulmod(twi[((size_t)(c.nq + k) << c.logn) + i].x, phi[k], q);
+            p_fold[2 * k + i].x = v;
+            p_fold[2 * k + i].y = H::shoup(v, q);
+        }
+        for (int l = 0; l < c.nq; l++) {
+            const uint64_t v = H::mulmod(phm[(size_t)l * c.np + k], pinv[l], Q[l]);
+            md_c[(size_t)l * c.np + k].x = neg(v, Q[l]);
+            md_c[(size_t)l * c.np + k].y = H::shoup(neg(v, Q[l]), Q[l]);
+        }
+    }
+    const size_t o_pf = blob.add(p_fold), o_mdc = blob.add(md_c);
     // T-base key switch constants (include/BasisConv.cuh:11-226; the reference's
     // precompute is in include/BFVcontext.cuh). Blocks lift by approximate CRT:
     // (B/b_j)^-1 mod b_j, B/b_j mod t_k and B mod t_k per block B.
@@ -519,6 +535,8 @@ void build_context(Context& c, const kbfv_params& prm) {
     dc.dig_vq_mod = U(o_ks[10]);
     dc.mm_q2r = base + o_mmq2r; dc.mm_sr = base + o_mmsr; dc.mm_r2q = base + o_mmr2q; dc.mm_lift = base + o_mmlift;
     dc.qr_fold = (const tw_t*)(base + o_qrf);
+    dc.p_fold = (const tw_t*)(base + o_pf);
+    dc.md_c = (const tw_t*)(base + o_mdc);
     dc.ms_qlinv = U(o_ms[0]); dc.ms_qlinvs = U(o_ms[1]); dc.ms_half_mod = U(o_ms[2]);
     dc.gauss_cdt = U(o_cdt);
     if (c.klss_ok) {

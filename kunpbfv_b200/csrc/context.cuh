@@ -69,6 +69,8 @@ struct DevConsts {
     uint64_t mm_lift_stride;
     const tw_t* qr_fold;  // [nqr][2]: the inverse NTT's last-stage constants over Q|R, those of an R prime
                           // times its scale-and-round constant and (R/r_j)^-1
+    const tw_t* p_fold;   // [np][2]: the inverse NTT's last-stage constants over P times (P/p_k)^-1 mod p_k
+    const tw_t* md_c;     // [nq][np]: -(P/p_k) P^-1 mod q_l
     int mm_ks;
     int mm_shift;  // 1: some prime of Q or R has fewer than 60 bits
     int key_nq, key_npq;         // limb layout of the relinearisation key (top level's Q and Q|P counts)

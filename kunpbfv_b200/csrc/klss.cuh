@@ -109,15 +109,29 @@ static __global__ void klss_t_to_pq_kernel(DevConsts c, KlssConsts kc, const uin
 // External product over T (NTT form), fused into the inverse NTT's load:
 // row (item, h, b, t): sum over digits i of dig[item][i][t] * key[h][i][b][t] mod t_t.
 struct ExtProdRow {
+    static constexpr bool kLoadMany = true;
     const uint64_t* dig;   // digit 0, T prime t
     const uint64_t* key;   // half h, digit 0, block b, T prime t
     size_t ds, ks;
     int ndig;
     uint64_t q, mh, ml;
-    __device__ __forceinline__ uint64_t load(int j) const {
-        u128 acc{0, 0};
-        for (int i = 0; i < ndig; i++) mac(acc, dig[i * ds + j], key[i * ks + j]);
-        return barrett128(acc, q, mh, ml);
+    template <int K>
+    __device__ __forceinline__ void load_n(const int (&j)[K], uint64_t* x) const {
+        u128 acc[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) acc[i] = u128{0, 0};
+        for (int d = 0; d < ndig; d++) {
+            uint64_t a[K], b[K];
+#pragma unroll
+            for (int i = 0; i < K; i++) {
+                a[i] = __ldg(dig + d * ds + j[i]);
+                b[i] = __ldg(key + d * ks + j[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < K; i++) mac(acc[i], a[i], b[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) x[i] = barrett128(acc[i], q, mh, ml);
     }
     __device__ __forceinline__ void store(int, uint64_t) const {}
 };

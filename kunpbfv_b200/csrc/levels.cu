@@ -178,10 +178,7 @@ static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& p
     // K7: mod down + add fused into NTT over Q, the key product over Q added at its store
     const StageRows r7 = stage_rows(G, [&](int g) { return 2 * G.nq[g]; }, &n);
     const MixedOutCtKeyDst dst{pb, m.sd2, rlk, G, r7};
-    if (G.np == 1)
-        ntt_fwd(dc, MixedModDownSrc<true>{m.se, m.sd, G, r7}, dst, n, st);
-    else
-        ntt_fwd(dc, MixedModDownSrc<false>{m.se, m.sd, G, r7}, dst, n, st);
+    ntt_fwd(dc, MixedModDownSrc{m.se, m.sd, G, r7}, dst, n, st);
 }
 
 extern "C" {

@@ -160,7 +160,6 @@ struct MixedTensorSrc {
         t.k = k;
         t.q = lv->mods[pi];
         t.mh = lv->mu_prod[pi];
-        t.ml = 0;
         if (l < nq) {
             const uint64_t* A = pb.a[L.item];
             const uint64_t* B = pb.b[L.item];
@@ -203,7 +202,7 @@ struct MixedKeyIPSrc {
     }
 };
 
-// K6b destination: the P limbs of se (item region of 2 x top_npq limbs, [2][npq] packed)
+// K6b destination: the P limbs of se (item region of 2 x top_npq limbs, [2][npq] packed; see SeFoldRowsP)
 struct MixedSeRowsP {
     uint64_t* se;
     Groups G;
@@ -219,11 +218,14 @@ struct MixedSeRowsP {
         const int h = (int)G.dp.div(L.local);
         return PtrRow{se + (((size_t)L.item * 2 * G.top_npq + h * G.npq[L.g] + limb(L)) << G.logn)};
     }
+    __device__ __forceinline__ const tw_t* fold(int row) const {
+        const RowLoc L = locate(G, R, row);
+        return G.lv[L.g]->p_fold + 2 * (int)G.dp.mod(L.local);
+    }
 };
 
-// K7 source: mod down of the P part and the add term (see ModDownAdd1Src /
-// ModDownAddSrc); rows (item, h, l), 2 x nq rows per item
-template <bool ONE_P>
+// K7 source: mod down of the P part and the add term (see ModDownKeySrc); rows
+// (item, h, l), 2 x nq rows per item
 struct MixedModDownSrc {
     const uint64_t* se;
     const uint64_t* sd;  // item region of 2 x top_nq limbs, [2][nq] packed
@@ -237,35 +239,18 @@ struct MixedModDownSrc {
         const RowLoc L = locate(G, R, row);
         return level_tab(G.lv[L.g], (int)G.dq[L.g].mod(L.local), inverse, G.logn);
     }
-    __device__ __forceinline__ auto bind(int row) const {
+    __device__ __forceinline__ ModDownKeyRow bind(int row) const {
         const RowLoc L = locate(G, R, row);
         const int g = L.g, nq = G.nq[g], logn = G.logn, h = (int)G.dq[g].div(L.local), l = L.local - h * nq;
         const DevConsts* lv = G.lv[g];
-        const uint64_t* poly = se + (((size_t)L.item * 2 * G.top_npq + (size_t)h * G.npq[g]) << logn);
-        const uint64_t* add = sd + (((size_t)L.item * 2 * G.top_nq + (size_t)h * nq + l) << logn);
-        if constexpr (ONE_P) {
-            ModDownAdd1Row r;
-            r.x = nullptr;  // the Q part is added in the NTT domain at K7's store
-            r.xp = poly + ((size_t)nq << logn);
-            r.add = add;
-            r.q = lv->mods[l]; r.mh = lv->mu_hi[l];
-            r.pinv = lv->pinv_q[l]; r.pinvs = lv->pinv_qs[l];
-            return r;
-        } else {
-            ModDownAddRow r;
-            r.x = nullptr;
-            r.xp = poly + ((size_t)nq << logn);
-            r.add = add;
-            r.pmods = lv->mods + lv->idx_p;
-            r.phatinv = lv->phatinv_p;
-            r.phatinvs = lv->phatinv_ps;
-            r.phat = lv->phat_mod_q + (size_t)l * lv->np;
-            r.limb = (size_t)1 << logn;
-            r.np = lv->np;
-            r.q = lv->mods[l]; r.mh = lv->mu_hi[l]; r.ml = lv->mu_lo[l];
-            r.pinv = lv->pinv_q[l]; r.pinvs = lv->pinv_qs[l];
-            return r;
-        }
+        ModDownKeyRow r;
+        r.xp = se + (((size_t)L.item * 2 * G.top_npq + (size_t)h * G.npq[g] + nq) << logn);
+        r.add = sd + (((size_t)L.item * 2 * G.top_nq + (size_t)h * nq + l) << logn);
+        r.c = lv->md_c + (size_t)l * lv->np;
+        r.limb = (size_t)1 << logn;
+        r.np = lv->np;
+        r.q = lv->mods[l];
+        return r;
     }
 };
 

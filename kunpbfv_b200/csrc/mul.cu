@@ -14,13 +14,9 @@
 //   NTT(add - P^-1 [x_P]_Q) + P^-1 x_Q,  with x_Q computed at the store.
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
                     const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st) {
-    ntt_inv(dc, KeyIPSrc{sd2, key, dc, ndig, dc.nq, dc.np}, SeRowsP{se, dc.logn, dc.nq, dc.np, dc.npq},
+    ntt_inv(dc, KeyIPSrc{sd2, key, dc, ndig, dc.nq, dc.np}, SeFoldRowsP{se, dc.logn, dc.nq, dc.np, dc.npq, dc.p_fold},
             count * 2 * dc.np, st);
-    const OutCtKeyDst dst{pb, sd2, key, dc, ndig};
-    if (dc.np == 1)
-        ntt_fwd(dc, ModDownAdd1Src{se, add, dc, true}, dst, count * 2 * dc.nq, st);
-    else
-        ntt_fwd(dc, ModDownAddSrc{se, add, dc, true}, dst, count * 2 * dc.nq, st);
+    ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtKeyDst{pb, sd2, key, dc, ndig}, count * 2 * dc.nq, st);
 }
 
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st) {

@@ -78,6 +78,38 @@ struct has_prefetch : std::false_type {};
 template <class T>
 struct has_prefetch<T, std::void_t<decltype(std::declval<const T&>().prefetch(0, 0, 0))>> : std::true_type {};
 
+// A row whose load or store computes from several operands can take several
+// points at once (`load_n<K>(j, x)`, `store_n<K>(j, v)` with v below 8q, not
+// reduced): all points' operands are then in flight together, where one point
+// after the other waits for memory K times (the compiler moves no load across a
+// store or a loop over the key switch's digits).
+template <class T, class = void>
+struct has_load_n : std::false_type {};
+template <class T>
+struct has_load_n<T, std::enable_if_t<T::kLoadMany>> : std::true_type {};
+template <class T, class = void>
+struct has_store_n : std::false_type {};
+template <class T>
+struct has_store_n<T, std::enable_if_t<T::kStoreMany>> : std::true_type {};
+
+// x[k] = row value at index(k), k < K
+template <int K, class Row, class Index>
+__device__ __forceinline__ void load_points(const Row& s, uint64_t* x, Index index) {
+    if constexpr (has_load_n<Row>::value) {
+        constexpr int C = K < 4 ? K : 4;
+#pragma unroll
+        for (int k = 0; k < K; k += C) {
+            int j[C];
+#pragma unroll
+            for (int i = 0; i < C; i++) j[i] = index(k + i);
+            s.template load_n<C>(j, x + k);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) x[k] = s.load(index(k));
+    }
+}
+
 // asynchronous copy of `bytes` (a multiple of 16, 16-byte aligned) into L2
 __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
@@ -417,8 +449,7 @@ __device__ __forceinline__ void inv_pass_load(const PassCtx& c, const SRow& s) {
     for (int g = 0; g < NG; g++) {
         const int lbase = adjacent_group<LOGB, R>(g, c.t) << R;
         uint64_t x[G];
-#pragma unroll
-        for (int k = 0; k < G; k++) x[k] = s.load(c.goff + lbase + k);
+        load_points<G>(s, x, [&](int k) { return c.goff + lbase + k; });
         const int s0 = c.sbase + S0;
         inv_group<R>(x, c.tw, s0, (c.goff + lbase) >> (c.logn - s0), c.q, c.q4, false);
 #pragma unroll
@@ -472,8 +503,7 @@ ntt_fwd_block_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const ui
     for (int g = 0; g < 16 / G0; g++) {
         const int gi = g * T + t;
         uint64_t x[G0];
-#pragma unroll
-        for (int k = 0; k < G0; k++) x[k] = s.load(c.goff + gi + (k << lb0));
+        load_points<G0>(s, x, [&](int k) { return c.goff + gi + (k << lb0); });
         fwd_group<R0>(x, c.tw, c.sbase, c.goff >> LOGB, q, q4);
         const int pg = spad(gi);
 #pragma unroll
@@ -485,11 +515,26 @@ ntt_fwd_block_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const ui
     // straight to the row measured 14% slower here); the store target is bound
     // here, so a fused store's operands hold no registers during the transform
     const auto d = dst.bind(row);
+    if constexpr (has_store_n<decltype(d)>::value) {
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const int j = sweep_index<LOGB>(t, k);
-        const uint64_t v = sm[spad(j)];
-        d.store(c.goff + j, FULL ? reduce_from(v, q, 3) : v);
+        for (int k = 0; k < 16; k += 4) {
+            int j[4];
+            uint64_t v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                j[i] = sweep_index<LOGB>(t, k + i);
+                v[i] = sm[spad(j[i])];
+                j[i] += c.goff;
+            }
+            d.template store_n<4>(j, v);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const int j = sweep_index<LOGB>(t, k);
+            const uint64_t v = sm[spad(j)];
+            d.store(c.goff + j, FULL ? reduce_from(v, q, 3) : v);
+        }
     }
 }
 
@@ -515,9 +560,11 @@ ntt_inv_block_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const ui
         inv_passes_load<LOGB, RAD, R0>(c, s);
     } else {
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const int j = sweep_index<LOGB>(t, k);
-            sm[spad(j)] = s.load(c.goff + j);
+        for (int k = 0; k < 16; k += 4) {
+            uint64_t x[4];
+            load_points<4>(s, x, [&](int i) { return c.goff + sweep_index<LOGB>(t, k + i); });
+#pragma unroll
+            for (int i = 0; i < 4; i++) sm[spad(sweep_index<LOGB>(t, k + i))] = x[i];
         }
         team_sync<LOGB>();
         inv_passes<LOGB, RAD, R0>(c);
@@ -554,8 +601,7 @@ __device__ __forceinline__ void ntt_fwd_col(const Src& src, const Dst& dst, cons
     const uint64_t q = rt.q, q4 = q << 2;
     const tw_t* tw = rt.tw;
     uint64_t x[1 << RC];
-#pragma unroll
-    for (int k = 0; k < (1 << RC); k++) x[k] = s.load(c + k * cols);
+    load_points<(1 << RC)>(s, x, [&](int k) { return c + k * cols; });
     fwd_group<RC>(x, tw, 0, 0, q, q4);
 #pragma unroll
     for (int k = 0; k < (1 << RC); k++) d.store(c + k * cols, x[k]);

@@ -45,16 +45,18 @@ struct QRFoldRowsIO {
 };
 
 // K4 source: tensor product of the pair at limb l of Q|R, one of three outputs
+// values in [0, 4q), as the inverse transform takes them; the loads are read-only ones: no store
+// of the kernel holds them back
 struct TensorRow {
     const uint64_t *a1, *b1, *a2, *b2;
     int k;
-    uint64_t q, mh, ml;  // mh: barrett_prod constant (inputs are fully reduced)
+    uint64_t q, mh;  // mh: barrett_prod constant (inputs are fully reduced)
     __device__ __forceinline__ uint64_t load(int j) const {
-        if (k == 0) return mul_mod_prod(a1[j], a2[j], q, mh);
-        if (k == 2) return mul_mod_prod(b1[j], b2[j], q, mh);
-        u128 acc = mul_wide(a1[j], b2[j]);
-        mac(acc, b1[j], a2[j]);  // < 2 q^2
-        return barrett_prod(acc, q, mh);
+        if (k == 0) return barrett_prod_lazy(mul_wide(__ldg(a1 + j), __ldg(a2 + j)), q, mh);
+        if (k == 2) return barrett_prod_lazy(mul_wide(__ldg(b1 + j), __ldg(b2 + j)), q, mh);
+        u128 acc = mul_wide(__ldg(a1 + j), __ldg(b2 + j));
+        mac(acc, __ldg(b1 + j), __ldg(a2 + j));  // < 2 q^2
+        return barrett_prod_lazy(acc, q, mh);
     }
     __device__ __forceinline__ void store(int, uint64_t) const {}
 };
@@ -72,7 +74,7 @@ struct TensorSrc {
         TensorRow t;
         t.k = k;
         const int pi = l < nq ? l : dc.idx_r + (l - nq);
-        t.q = dc.mods[pi]; t.mh = dc.mu_prod[pi]; t.ml = 0;
+        t.q = dc.mods[pi]; t.mh = dc.mu_prod[pi];
         if (l < nq) {
             const uint64_t* A = pb.a[item];
             const uint64_t* B = pb.b[item];
@@ -88,18 +90,52 @@ struct TensorSrc {
     }
 };
 
+// sum_d digit_d * key_d at K points: [0, 4q) for one digit (fully reduced
+// factors), else [0, q). All points' operands of a digit are loaded before they
+// are used, by read-only loads.
+template <int K>
+__device__ __forceinline__ void key_product(const uint64_t* dig, const uint64_t* key, size_t ds, size_t ks, int ndig,
+                                            uint64_t q, uint64_t mh, uint64_t ml, uint64_t mp, const int (&j)[K],
+                                            uint64_t* x) {
+    uint64_t a[K], b[K];
+    if (ndig == 1) {
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            a[i] = __ldg(dig + j[i]);
+            b[i] = __ldg(key + j[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) x[i] = barrett_prod_lazy(mul_wide(a[i], b[i]), q, mp);
+        return;
+    }
+    u128 acc[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) acc[i] = u128{0, 0};
+    for (int d = 0; d < ndig; d++, dig += ds, key += ks) {
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            a[i] = __ldg(dig + j[i]);
+            b[i] = __ldg(key + j[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) mac(acc[i], a[i], b[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < K; i++) x[i] = barrett128(acc[i], q, mh, ml);
+}
+
 // K6b source: inner product with the relinearisation key over Q|P
 struct KeyIPRow {
+    static constexpr bool kLoadMany = true;
     const uint64_t* dig;  // limb m of digit 0 (digit stride ds)
     const uint64_t* key;  // limb m, half h of digit 0 (digit stride ks)
     size_t ds, ks;
     int dnum;
     uint64_t q, mh, ml, mp;
-    __device__ __forceinline__ uint64_t load(int j) const {
-        if (dnum == 1) return mul_mod_prod(dig[j], key[j], q, mp);  // digits fully reduced
-        u128 acc{0, 0};
-        for (int d = 0; d < dnum; d++) mac(acc, dig[d * ds + j], key[d * ks + j]);
-        return barrett128(acc, q, mh, ml);
+    // [0, 4q) (one digit) or [0, q)
+    template <int K>
+    __device__ __forceinline__ void load_n(const int (&j)[K], uint64_t* x) const {
+        key_product<K>(dig, key, ds, ks, dnum, q, mh, ml, mp, j, x);
     }
     __device__ __forceinline__ void store(int, uint64_t) const {}
 };
@@ -152,9 +188,9 @@ struct GadgetDigitSrc {
     }
 };
 
-// K7 source: mod down P|Q -> q_l and add the tensor term (coefficient form)
+// K7 source of the T-base key switch: mod down P|Q -> q_l and add the tensor term (coefficient form)
 struct ModDownAddRow {
-    const uint64_t* x;    // limb l of the Q|P polynomial, or null (Q part added in the NTT domain)
+    const uint64_t* x;    // limb l of the Q|P polynomial
     const uint64_t* xp;   // limb 0 of its P part
     const uint64_t* add;  // limb l of the term to add, or null
     const uint64_t* pmods;
@@ -176,7 +212,7 @@ struct ModDownAddRow {
             }
             conv = barrett128(acc, q, mh, ml);
         }
-        uint64_t v = shoup(q - conv + (x ? x[j] : 0), pinv, pinvs, q);
+        uint64_t v = shoup(q - conv + x[j], pinv, pinvs, q);
         if (add) v = add_mod(v, add[j], q);
         return v;
     }
@@ -186,14 +222,13 @@ struct ModDownAddSrc {
     const uint64_t* se;   // [item][2][npq]
     const uint64_t* sd;   // [item][2][nq] or null
     DevConsts dc;
-    bool p_only = false;  // se holds only the P limbs (OutCtKeyDst adds the Q part)
     __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
     __device__ __forceinline__ ModDownAddRow bind(int row) const {
         const int nq = dc.nq, npq = dc.npq, logn = dc.logn;
         const int item = row / (2 * nq), w = row % (2 * nq), h = w / nq, l = w % nq;
         ModDownAddRow r;
         const uint64_t* poly = se + (((size_t)item * 2 + h) * npq << logn);
-        r.x = p_only ? nullptr : poly + ((size_t)l << logn);
+        r.x = poly + ((size_t)l << logn);
         r.xp = poly + ((size_t)nq << logn);
         r.add = sd ? sd + (((size_t)(item * 2 + h) * nq + l) << logn) : nullptr;
         r.pmods = dc.mods + dc.idx_p;
@@ -208,37 +243,56 @@ struct ModDownAddSrc {
     }
 };
 
-// ModDownAddSrc for one special prime: [x_P]_q is x_P mod q, so the row needs
-// no conversion tables (fewer live registers in the transform's first pass)
-struct ModDownAdd1Row {
-    const uint64_t* x;    // limb l of the Q|P polynomial, or null
-    const uint64_t* xp;   // its P limb
+// K7 source of the key-switch tail: add - P^-1 [x_P]_q over Q. K6b stores the P
+// limbs as rb_k = [x_k (P/p_k)^-1]_{p_k} (SeFoldRowsP), so that
+//   P^-1 [x_P]_q = sum_k rb_k (P/p_k) P^-1  mod q
+// is one lazy Shoup product per special prime with the constants
+// md_c = -(P/p_k) P^-1 mod q: the reduction of every P limb for every prime of Q
+// (and a 128-bit Barrett reduction and a product by P^-1) took 2.5 times the
+// multiplies at two special primes. Values below 5q.
+struct ModDownKeyRow {
+    static constexpr bool kLoadMany = true;
+    const uint64_t* xp;   // P limb 0
     const uint64_t* add;  // limb l of the term to add, or null
-    uint64_t q, mh, pinv, pinvs;
-    __device__ __forceinline__ uint64_t load(int j) const {
-        const uint64_t conv = barrett64(xp[j], q, mh);
-        uint64_t v = shoup(q - conv + (x ? x[j] : 0), pinv, pinvs, q);
-        if (add) v = add_mod(v, add[j], q);
-        return v;
+    const tw_t* c;        // md_c of prime l: [np], with Shoup companions
+    size_t limb;
+    int np;
+    uint64_t q;
+    template <int K>
+    __device__ __forceinline__ void load_n(const int (&j)[K], uint64_t* x) const {
+        uint64_t y[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            y[i] = __ldg(xp + j[i]);
+            x[i] = add ? __ldg(add + j[i]) : 0;
+        }
+        for (int k = 0; k < np; k++) {
+            if (k) {
+#pragma unroll
+                for (int i = 0; i < K; i++) y[i] = __ldg(xp + k * limb + j[i]);
+            }
+            const ulonglong2 w = __ldg(c + k);
+#pragma unroll
+            for (int i = 0; i < K; i++) x[i] = csub63(x[i], q << 2) + shoup4(y[i], w.x, w.y, q);
+        }
     }
     __device__ __forceinline__ void store(int, uint64_t) const {}
 };
-struct ModDownAdd1Src {
-    const uint64_t* se;   // [item][2][npq]
+struct ModDownKeySrc {
+    const uint64_t* se;   // [item][2][npq], P limbs scaled
     const uint64_t* sd;   // [item][2][nq] or null
     DevConsts dc;
-    bool p_only = false;
     __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
-    __device__ __forceinline__ ModDownAdd1Row bind(int row) const {
-        const int nq = dc.nq, npq = dc.npq, logn = dc.logn;
+    __device__ __forceinline__ ModDownKeyRow bind(int row) const {
+        const int nq = dc.nq, logn = dc.logn;
         const int item = row / (2 * nq), w = row % (2 * nq), h = w / nq, l = w % nq;
-        const uint64_t* poly = se + (((size_t)item * 2 + h) * npq << logn);
-        ModDownAdd1Row r;
-        r.x = p_only ? nullptr : poly + ((size_t)l << logn);
-        r.xp = poly + ((size_t)nq << logn);
+        ModDownKeyRow r;
+        r.xp = se + ((((size_t)item * 2 + h) * dc.npq + nq) << logn);
         r.add = sd ? sd + (((size_t)(item * 2 + h) * nq + l) << logn) : nullptr;
-        r.q = dc.mods[l]; r.mh = dc.mu_hi[l];
-        r.pinv = dc.pinv_q[l]; r.pinvs = dc.pinv_qs[l];
+        r.c = dc.md_c + (size_t)l * dc.np;
+        r.limb = (size_t)1 << logn;
+        r.np = dc.np;
+        r.q = dc.mods[l];
         return r;
     }
 };
@@ -253,37 +307,38 @@ struct OutCtDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
     }
 };
 
-// rows (item, h, k) -> limb nq + k (P part) of se ([item][2][npq])
-struct SeRowsP {
+// rows (item, h, k) -> limb nq + k (P part) of se ([item][2][npq]), stored times
+// (P/p_k)^-1 mod p_k (folded into the inverse transform's last-stage constants)
+struct SeFoldRowsP {
     uint64_t* se;
     int logn, nq, np, npq;
+    const tw_t* fold_base;  // DevConsts::p_fold
     __device__ __forceinline__ int prime(int row) const { return nq + row % np; }
     __device__ __forceinline__ PtrRow bind(int row) const {
         const int item = row / (2 * np), w = row % (2 * np), h = w / np, k = w % np;
         return PtrRow{se + (((size_t)(item * 2 + h) * npq + nq + k) << logn)};
     }
+    __device__ __forceinline__ const tw_t* fold(int row) const { return fold_base + 2 * (row % np); }
 };
 
 // Output store of the key-switch tail: adds P^-1 * sum_d digit_d * key_d[h] at
 // limb l of Q (all NTT form, fully reduced) to the transformed value.
 struct OutKeyRow {
+    static constexpr bool kStoreMany = true;
     uint64_t* p;
     const uint64_t* dig;  // limb l of digit 0, digit stride ds
     const uint64_t* key;  // limb l of half h of digit 0, digit stride ks
     size_t ds, ks;
     int ndig;
     uint64_t q, mh, ml, mp, pinv, pinvs;
-    __device__ __forceinline__ uint64_t load(int j) const { return p[j]; }
-    __device__ __forceinline__ void store(int j, uint64_t v) const {
-        uint64_t ip;
-        if (ndig == 1) {
-            ip = mul_mod_prod(dig[j], key[j], q, mp);
-        } else {
-            u128 acc{0, 0};
-            for (int d = 0; d < ndig; d++) mac(acc, dig[d * ds + j], key[d * ks + j]);
-            ip = barrett128(acc, q, mh, ml);
-        }
-        p[j] = add_mod(v, shoup(ip, pinv, pinvs, q), q);
+    // v below 8q
+    template <int K>
+    __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
+        uint64_t ip[K];
+        key_product<K>(dig, key, ds, ks, ndig, q, mh, ml, mp, j, ip);
+#pragma unroll
+        for (int i = 0; i < K; i++)
+            p[j[i]] = reduce_from(csub63(v[i], q << 2) + shoup4(ip[i], pinv, pinvs, q), q, 3);
     }
 };
 struct OutCtKeyDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
@@ -331,8 +386,10 @@ struct DecSrc {
     struct Row {
         const uint64_t *a, *b, *s;
         uint64_t q, mh, ml;
-        // a and s fully reduced: one-high-product Barrett (mh holds its constant)
-        __device__ __forceinline__ uint64_t load(int j) const { return add_mod(mul_mod_prod(a[j], s[j], q, mh), b[j], q); }
+        // a and s fully reduced: one-high-product Barrett (mh holds its constant); below 3q
+        __device__ __forceinline__ uint64_t load(int j) const {
+            return csub63(barrett_prod_lazy(mul_wide(__ldg(a + j), __ldg(s + j)), q, mh), q << 1) + __ldg(b + j);
+        }
         __device__ __forceinline__ void store(int, uint64_t) const {}
     };
     __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }

@@ -112,7 +112,9 @@ struct DecSrcP {
     struct Row {
         const uint64_t *a, *b, *s;
         uint64_t q, mp;
-        __device__ __forceinline__ uint64_t load(int j) const { return add_mod(mul_mod_prod(a[j], s[j], q, mp), b[j], q); }
+        __device__ __forceinline__ uint64_t load(int j) const {  // below 3q, as DecSrc
+            return csub63(barrett_prod_lazy(mul_wide(__ldg(a + j), __ldg(s + j)), q, mp), q << 1) + __ldg(b + j);
+        }
         __device__ __forceinline__ void store(int, uint64_t) const {}
     };
     __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
