@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -76,6 +77,21 @@ static inline unsigned blocks_for(size_t total, unsigned threads) { return (unsi
 // grid of a grid-stride kernel: enough blocks to cover `total`, at most 2^20
 static inline unsigned stride_blocks(size_t total, unsigned threads) {
     return (unsigned)std::min<size_t>((total + threads - 1) / threads, (size_t)1 << 20);
+}
+
+static inline bool aligned16(std::initializer_list<const void*> ps) {
+    uintptr_t x = 0;
+    for (const void* p : ps) x |= (uintptr_t)p;
+    return (x & 15) == 0;
+}
+// out = x + y over `items` items of `per` rows of N words (limb = row % limbs), item strides in words
+static inline void launch_add(const DevConsts& dc, const uint64_t* x, size_t xs, const uint64_t* y, size_t ys,
+                              uint64_t* out, size_t os, size_t items, int per, int limbs, cudaStream_t st) {
+    if (aligned16({x, y, out}))
+        add_kernel<2><<<row_blocks<2>(items * per, dc.logn), 256, 0, st>>>(dc, x, xs, y, ys, out, os, per, limbs);
+    else
+        add_kernel<1><<<row_blocks<1>(items * per, dc.logn), 256, 0, st>>>(dc, x, xs, y, ys, out, os, per, limbs);
+    check_launch("add");
 }
 
 // CTAs of `kernel` that fit on the device at once (SMs x CTAs per SM)

@@ -276,10 +276,43 @@ static __global__ void decrypt_round_kernel(DevConsts c, const uint64_t* __restr
 // limb-wise arithmetic. Index space: items x polys x limbs x N; the prime of a
 // limb is prime0 + limb.
 // ===========================================================================
-struct LimbIdx {
-    int logn, limbs;
-    __device__ __forceinline__ int limb(size_t i) const { return (int)((i >> logn) % (size_t)limbs); }
+// The kernels run over rows of N words: a CTA of 256 threads takes 256 V
+// consecutive words of one row (V = 2: 16-byte accesses, where every pointer is
+// 16-byte aligned), so a row's item, limb and constants are found once per
+// thread in 32-bit arithmetic. With a 64-bit division and remainder per word
+// instead, a plaintext product of 7 ciphertexts at N = 32768 took 52 us for
+// 147 MB, now 34 us.
+template <int V>
+struct Words {
+    uint64_t v[V];
 };
+template <int V>
+__device__ __forceinline__ Words<V> load_words(const uint64_t* p) {
+    if constexpr (V == 2) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p);
+        return Words<2>{{x.x, x.y}};
+    } else {
+        return Words<1>{{*p}};
+    }
+}
+template <int V>
+__device__ __forceinline__ void store_words(uint64_t* p, const Words<V>& w) {
+    if constexpr (V == 2) *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(w.v[0], w.v[1]);
+    else *p = w.v[0];
+}
+struct RowAt {
+    unsigned row;
+    size_t j;  // word in the row
+};
+template <int V>
+__device__ __forceinline__ RowAt row_at(int logn) {
+    const int lc = logn - (V == 2 ? 9 : 8);
+    return RowAt{blockIdx.x >> lc, ((size_t)(blockIdx.x & ((1u << lc) - 1)) * 256 + threadIdx.x) * V};
+}
+template <int V>
+static inline unsigned row_blocks(size_t rows, int logn) {
+    return (unsigned)(rows << (logn - (V == 2 ? 9 : 8)));
+}
 
 // ceil(Q*m/t) per limb (bfv_add_timesQ_overt_kernel, include/poly_arithmetic.cuh:902-927)
 static __global__ void delta_m_kernel(DevConsts c, const uint64_t* __restrict__ m, uint64_t* __restrict__ out, size_t total) {
@@ -293,12 +326,19 @@ static __global__ void delta_m_kernel(DevConsts c, const uint64_t* __restrict__ 
     out[i] = shoup(mq, c.tinv_q[l], c.tinv_qs[l], c.mods[l]);
 }
 
-static __global__ void add_kernel(DevConsts c, const uint64_t* __restrict__ x, const uint64_t* __restrict__ y,
-                           uint64_t* __restrict__ out, size_t total, int limbs) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const int l = (int)((i >> c.logn) % limbs);
-    out[i] = add_mod(x[i], y[i], c.mods[l]);
+// out = x + y over items of `per` rows (limb = row % limbs), item strides in words
+template <int V>
+static __global__ void add_kernel(DevConsts c, const uint64_t* x, size_t xs, const uint64_t* y, size_t ys,
+                                  uint64_t* out, size_t os, int per, int limbs) {
+    const RowAt r = row_at<V>(c.logn);
+    const unsigned item = r.row / per, w = r.row % per;
+    const size_t at = ((size_t)w << c.logn) + r.j;
+    const uint64_t q = c.mods[w % limbs];
+    Words<V> a = load_words<V>(x + item * xs + at);
+    const Words<V> b = load_words<V>(y + item * ys + at);
+#pragma unroll
+    for (int i = 0; i < V; i++) a.v[i] = add_mod(a.v[i], b.v[i], q);
+    store_words<V>(out + item * os + at, a);
 }
 
 // limb-wise linear ops over ciphertexts (rows of N, limb = row % limbs):
@@ -307,30 +347,38 @@ static __global__ void add_kernel(DevConsts c, const uint64_t* __restrict__ x, c
 struct ScalarTab {
     uint64_t c[kMaxQ], cs[kMaxQ];
 };
-static __global__ void linear_kernel(DevConsts c, const uint64_t* x, const uint64_t* y, uint64_t* out, size_t total,
-                              int limbs, int op, ScalarTab tab) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const int l = (int)((i >> c.logn) % limbs);
+template <int V>
+static __global__ void linear_kernel(DevConsts c, const uint64_t* x, const uint64_t* y, uint64_t* out, int limbs, int op,
+                                     ScalarTab tab) {
+    const RowAt r = row_at<V>(c.logn);
+    const int l = (int)(r.row % limbs);
+    const size_t at = ((size_t)r.row << c.logn) + r.j;
     const uint64_t q = c.mods[l];
-    uint64_t v;
-    if (op == 0) v = sub_mod(x[i], y[i], q);
-    else if (op == 1) v = x[i] ? q - x[i] : 0;
-    else if (op == 2) v = shoup(x[i], tab.c[l], tab.cs[l], q);
-    else v = add_mod(y[i], shoup(x[i], tab.c[l], tab.cs[l], q), q);
-    out[i] = v;
+    Words<V> a = load_words<V>(x + at), b{};
+    if (op == 0 || op == 3) b = load_words<V>(y + at);
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+        uint64_t& v = a.v[i];
+        if (op == 0) v = sub_mod(v, b.v[i], q);
+        else if (op == 1) v = v ? q - v : 0;
+        else if (op == 2) v = shoup(v, tab.c[l], tab.cs[l], q);
+        else v = add_mod(b.v[i], shoup(v, tab.c[l], tab.cs[l], q), q);
+    }
+    store_words<V>(out + at, a);
 }
 
 // ct (items x 2 x nq) times pt (items x nq)
-static __global__ void mul_plain_kernel(DevConsts c, const uint64_t* __restrict__ ct, const uint64_t* __restrict__ pt,
-                                 uint64_t* __restrict__ out, size_t total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const size_t lq = (size_t)c.nq << c.logn;
-    const int l = (int)((i >> c.logn) % c.nq);
-    const size_t item = i / (2 * lq);
-    const uint64_t p = pt[item * lq + (i % lq)];
-    out[i] = mul_mod(ct[i], p, c.mods[l], c.mu_hi[l], c.mu_lo[l]);
+template <int V>
+static __global__ void mul_plain_kernel(DevConsts c, const uint64_t* ct, const uint64_t* pt, uint64_t* out) {
+    const RowAt r = row_at<V>(c.logn);
+    const int l = (int)(r.row % c.nq);
+    const size_t item = r.row / (2 * c.nq), at = ((size_t)r.row << c.logn) + r.j;
+    const uint64_t q = c.mods[l], mh = c.mu_hi[l], ml = c.mu_lo[l];
+    Words<V> a = load_words<V>(ct + at);
+    const Words<V> p = load_words<V>(pt + ((item * c.nq + l) << c.logn) + r.j);
+#pragma unroll
+    for (int i = 0; i < V; i++) a.v[i] = mul_mod(a.v[i], p.v[i], q, mh, ml);
+    store_words<V>(out + at, a);
 }
 
 // tensor over Q|R for the C-ABI building block: pairs of [a|b] (nqr limbs each)
@@ -470,21 +518,6 @@ static __global__ void sample_small_kernel(DevConsts c, SalsaKey key, uint64_t i
     if (gid >= per_item * items) return;
     const size_t item = gid / per_item, b = gid % per_item;
     sample_small_block<KIND>(c, key, id0 + item, b, prime0, limbs, out + item * item_stride);
-}
-
-// the same with one stream id per item (ids passed by value)
-struct IdTable {
-    uint64_t v[128];
-};
-template <int KIND>
-static __global__ void sample_small_ids_kernel(DevConsts c, SalsaKey key, IdTable ids, int prime0, int limbs,
-                                        uint64_t* __restrict__ out, size_t item_stride, int items) {
-    constexpr int PER = KIND == 0 ? 16 : 8;
-    const size_t per_item = ((size_t)1 << c.logn) / PER;
-    const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= per_item * items) return;
-    const size_t item = gid / per_item, b = gid % per_item;
-    sample_small_block<KIND>(c, key, ids.v[item], b, prime0, limbs, out + item * item_stride);
 }
 
 // Hamming-weight-h ternary secret (convert_HWT, include/Sampler_impl.cuh:68-87):
@@ -636,6 +669,14 @@ static __global__ void galois_ntt_kernel(DevConsts c, const uint64_t* __restrict
     const uint32_t i = (uint32_t)(x & (((size_t)1 << c.logn) - 1));
     out[x] = in[(row << c.logn) + galois_perm(i, g, c.logn)];
 }
+// rows (item, limb) of the b-parts of ciphertexts, permuted: out[item][l] = galois(ct[item][1][l])
+static __global__ void galois_b_kernel(const uint64_t* __restrict__ ct, uint64_t* __restrict__ out, uint64_t g, int logn,
+                                       int nq) {
+    const RowAt r = row_at<1>(logn);
+    const unsigned item = r.row / nq, l = r.row % nq;
+    out[((size_t)r.row << logn) + r.j] =
+        ct[(((size_t)item * 2 + 1) * nq + l << logn) + galois_perm((uint32_t)r.j, g, logn)];
+}
 // key-switch key component for a target polynomial t (NTT form over Q|P):
 // b = e - a*s + [l in digit] * P * t
 static __global__ void ksk_combine_kernel(DevConsts c, const uint64_t* __restrict__ a, const uint64_t* __restrict__ s,
@@ -649,22 +690,6 @@ static __global__ void ksk_combine_kernel(DevConsts c, const uint64_t* __restric
     const int lo = digit * c.alpha, hi = min(lo + c.alpha, c.nq);
     if (l >= lo && l < hi) v = add_mod(v, mul_mod(target[i], c.p_mod_q[l], q, mh, ml), q);
     eb[i] = v;
-}
-
-// encrypt: a = v*pk.a + e0, b = v*pk.b + e1 + dm (encryptZero/encryptMsg,
-// include/BFVScheme.cuh:87-146). work: items x [v | e0 | e1 | dm] x nq (NTT form)
-static __global__ void enc_combine_kernel(DevConsts c, const uint64_t* __restrict__ pk, const uint64_t* __restrict__ work,
-                                   uint64_t* __restrict__ ct, size_t total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;  // items * nq * N
-    const size_t lq = (size_t)c.nq << c.logn;
-    const size_t item = i / lq, w = i % lq;
-    const int l = (int)(w >> c.logn);
-    const uint64_t q = c.mods[l], mh = c.mu_hi[l], ml = c.mu_lo[l];
-    const uint64_t* wk = work + item * 4 * lq;
-    const uint64_t v = wk[w], e0 = wk[lq + w], e1 = wk[2 * lq + w], dm = wk[3 * lq + w];
-    ct[item * 2 * lq + w] = add_mod(mul_mod(v, pk[w], q, mh, ml), e0, q);
-    ct[item * 2 * lq + lq + w] = add_mod(add_mod(mul_mod(v, pk[lq + w], q, mh, ml), e1, q), dm, q);
 }
 
 }  // namespace kbfv

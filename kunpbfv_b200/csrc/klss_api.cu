@@ -149,12 +149,7 @@ int kbfv_relinearize_klss(kbfv_context* ctx, const uint64_t* d_rlk_t, const uint
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }
             PtrBatch pb = make_batch(Z.data(), Z.data(), O.data(), cnt);
             ntt_fwd(dc, ModDownAddSrc{m.se, nullptr, dc}, OutCtDst{pb, dc.logn, dc.nq}, cnt * 2 * dc.nq, st);
-            for (int i = 0; i < cnt; i++) {
-                const size_t tot = 2 * lq;
-                add_kernel<<<blocks_for(tot, 256), 256, 0, st>>>(dc, out + (size_t)i * 2 * lq, tz + (size_t)i * 3 * lq + lq,
-                                                                 out + (size_t)i * 2 * lq, tot, dc.nq);
-            }
-            check_launch("relin_add");
+            launch_add(dc, out, 2 * lq, tz + lq, 3 * lq, out, 2 * lq, (size_t)cnt, 2 * dc.nq, dc.nq, st);
         }
     });
 }

@@ -39,20 +39,36 @@ struct ModSwitchSrc {  // rows (poly, i < nq-1)
         return r;
     }
 };
-// out[poly][i] = (ct[poly][i] - corr[poly][i]) * q_last^-1 mod q_i
-__global__ void mod_switch_combine_kernel(DevConsts c, const uint64_t* __restrict__ ct,
-                                          const uint64_t* __restrict__ corr, uint64_t* __restrict__ out,
-                                          size_t total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const int nout = c.nq - 1;
-    const size_t row = i >> c.logn, j = i & (((size_t)1 << c.logn) - 1);
-    const size_t poly = row / nout;
-    const int l = (int)(row % nout);
-    const uint64_t q = c.mods[l];
-    const uint64_t x = ct[((poly * c.nq + l) << c.logn) + j];
-    out[i] = shoup(x + q - corr[i], c.ms_qlinv[l], c.ms_qlinvs[l], q);
-}
+// store target: out[poly][i] = (ct[poly][i] - correction) * q_last^-1 mod q_i (as
+// a kernel of its own, with the corrections written and read back, 30 of the
+// 144 us of a switch of 7 ciphertexts at N = 32768, 14 primes)
+struct ModSwitchOutRow {
+    static constexpr bool kStoreMany = true;
+    const uint64_t* ct;
+    uint64_t* out;
+    uint64_t q, w, ws;
+    // v below 8q
+    template <int K>
+    __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
+        uint64_t x[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) x[i] = __ldg(ct + j[i]);
+#pragma unroll
+        for (int i = 0; i < K; i++) out[j[i]] = shoup(x[i] + (q << 3) - v[i], w, ws, q);
+    }
+};
+struct ModSwitchDst {  // rows (poly, i < nq - 1)
+    const uint64_t* ct;
+    uint64_t* out;
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % (dc.nq - 1); }
+    __device__ __forceinline__ ModSwitchOutRow bind(int row) const {
+        const int nout = dc.nq - 1, poly = row / nout, i = row % nout;
+        return ModSwitchOutRow{ct + (((size_t)poly * dc.nq + i) << dc.logn), out + ((size_t)row << dc.logn), dc.mods[i],
+                               dc.ms_qlinv[i], dc.ms_qlinvs[i]};
+    }
+};
+static inline RowsIO plain_of(const ModSwitchDst& d) { return RowsIO{d.out, d.dc.logn, 0, d.dc.nq - 1}; }
 
 // rows (item, l) of the a-part of ciphertexts, read through the Galois permutation
 struct GaloisRow {
@@ -244,15 +260,11 @@ int kbfv_mod_switch(kbfv_context* ctx, const uint64_t* d_ct, uint64_t* d_out, ui
         for (uint32_t off = 0; off < count; off += chunk) {
             const int cnt = (int)std::min<uint32_t>(chunk, count - off);
             const int polys = cnt * 2;
-            uint64_t* last = (uint64_t*)ensure_scratch(c, (size_t)polys * (1 + nout) * c.n * 8);
-            uint64_t* corr = last + ((size_t)polys << c.logn);
+            uint64_t* last = (uint64_t*)ensure_scratch(c, (size_t)polys * c.n * 8);
             const uint64_t* in = d_ct + (size_t)off * 2 * c.nq * c.n;
             uint64_t* o = d_out + (size_t)off * 2 * nout * c.n;
             ntt_inv(dc, LastLimbSrc{in, c.logn, c.nq}, rows_io(dc, last, c.nq - 1, 1), polys, st);
-            ntt_fwd(dc, ModSwitchSrc{last, dc}, rows_io(dc, corr, 0, nout), polys * nout, st);
-            const size_t total = (size_t)polys * nout * c.n;
-            mod_switch_combine_kernel<<<stride_blocks(total, 256), 256, 0, st>>>(dc, in, corr, o, total);
-            check_launch("mod_switch");
+            ntt_fwd(dc, ModSwitchSrc{last, dc}, ModSwitchDst{in, o, dc}, polys * nout, st);
         }
     });
 }
@@ -340,13 +352,13 @@ static int gadget_chunk(const Context& c, int w) {
 }
 
 static void gadget_keyswitch(Context& c, const uint64_t* gk, int w, int count, const MulScratch& m, uint64_t* sg,
-                             const uint64_t* add, const PtrBatch& pb, cudaStream_t st) {
+                             const uint64_t* add, const PtrBatch& pb, cudaStream_t st, const KsExtra& ex = {}) {
     const DevConsts& dc = c.dc;
     const int J = gadget_pieces(w), ndig = c.nq * J;
     // fully reduced NTT outputs: the key product sums ndig terms below q^2
     ntt_fwd<GadgetDigitSrc, RowsIO, true>(dc, GadgetDigitSrc{m.sd2, dc, J, w}, rows_io(dc, sg, 0, dc.npq),
                                          count * ndig * dc.npq, st);
-    ks_tail(dc, sg, gk, ndig, m.se, add, pb, count, st);
+    ks_tail(dc, sg, gk, ndig, m.se, add, pb, count, st, ex);
 }
 
 int kbfv_relinearize_gadget(kbfv_context* ctx, const uint64_t* d_gk, uint32_t log_base, const uint64_t* d_tensor,
@@ -375,13 +387,7 @@ int kbfv_relinearize_gadget(kbfv_context* ctx, const uint64_t* d_gk, uint32_t lo
             std::vector<const uint64_t*> Z(cnt);
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }
             PtrBatch pb = make_batch(Z.data(), Z.data(), O.data(), cnt);
-            gadget_keyswitch(c, d_gk, w, cnt, m, sg, nullptr, pb, st);
-            for (int i = 0; i < cnt; i++) {
-                const size_t tot = 2 * lq;
-                add_kernel<<<blocks_for(tot, 256), 256, 0, st>>>(dc, out + (size_t)i * 2 * lq, tz + (size_t)i * 3 * lq + lq,
-                                                                 out + (size_t)i * 2 * lq, tot, dc.nq);
-            }
-            check_launch("relin_add");
+            gadget_keyswitch(c, d_gk, w, cnt, m, sg, nullptr, pb, st, KsExtra{tz + lq, 3 * lq, 0});
         }
     });
 }
@@ -437,9 +443,7 @@ int kbfv_apply_galois(kbfv_context* ctx, const uint64_t* d_gk, uint64_t galois_e
             const uint64_t* in = d_ct + (size_t)off * 2 * lq;
             uint64_t* out = d_out + (size_t)off * 2 * lq;
             // g(b) first (the output may overwrite the input): sb holds [item][nq]
-            for (int i = 0; i < cnt; i++)
-                galois_ntt_kernel<<<blocks_for(lq, 256), 256, 0, st>>>(dc, in + (size_t)i * 2 * lq + lq,
-                                                                        m.sb + (size_t)i * lq, galois_elt, lq);
+            galois_b_kernel<<<row_blocks<1>((size_t)cnt * c.nq, c.logn), 256, 0, st>>>(in, m.sb, galois_elt, c.logn, c.nq);
             check_launch("galois_b");
             // g(a) read through the permutation by the inverse NTT, then the hybrid key switch
             ntt_inv(dc, GaloisASrc{in, galois_elt, dc.logn, dc.nq}, digit_rows(dc, m.sd2), cnt * dc.nq, st);
@@ -450,11 +454,7 @@ int kbfv_apply_galois(kbfv_context* ctx, const uint64_t* d_gk, uint64_t galois_e
             std::vector<const uint64_t*> Z(cnt);
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }
             PtrBatch pb = make_batch(Z.data(), Z.data(), O.data(), cnt);
-            ks_tail(dc, m.sd2, d_gk, dc.dnum, m.se, nullptr, pb, cnt, st);
-            for (int i = 0; i < cnt; i++)
-                add_kernel<<<blocks_for(lq, 256), 256, 0, st>>>(dc, out + (size_t)i * 2 * lq + lq, m.sb + (size_t)i * lq,
-                                                                out + (size_t)i * 2 * lq + lq, lq, dc.nq);
-            check_launch("galois_add");
+            ks_tail(dc, m.sd2, d_gk, dc.dnum, m.se, nullptr, pb, cnt, st, KsExtra{m.sb, lq, 1});
         }
     });
 }

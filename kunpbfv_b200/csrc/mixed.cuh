@@ -302,6 +302,7 @@ struct MixedOutCtKeyDst {
         r.ndig = G.dnum[g];
         r.q = lv->mods[l]; r.mh = lv->mu_hi[l]; r.ml = lv->mu_lo[l]; r.mp = lv->mu_prod[l];
         r.pinv = lv->pinv_q[l]; r.pinvs = lv->pinv_qs[l];
+        r.extra = nullptr;
         return r;
     }
 };

@@ -13,10 +13,10 @@
 // stay in the NTT domain, where the forward NTT's store adds them:
 //   NTT(add - P^-1 [x_P]_Q) + P^-1 x_Q,  with x_Q computed at the store.
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
-                    const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st) {
+                    const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st, const KsExtra& ex) {
     ntt_inv(dc, KeyIPSrc{sd2, key, dc, ndig, dc.nq, dc.np}, SeFoldRowsP{se, dc.logn, dc.nq, dc.np, dc.npq, dc.p_fold},
             count * 2 * dc.np, st);
-    ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtKeyDst{pb, sd2, key, dc, ndig}, count * 2 * dc.nq, st);
+    ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtKeyDst{pb, sd2, key, dc, ndig, ex}, count * 2 * dc.nq, st);
 }
 
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st) {
@@ -121,14 +121,8 @@ int kbfv_relinearize(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_t* d
             std::vector<const uint64_t*> Z(cnt);
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }
             PtrBatch pb = make_batch(Z.data(), Z.data(), O.data(), cnt);
-            ks_tail(dc, m.sd2, d_rlk, dc.dnum, m.se, nullptr, pb, cnt, st);
-            // add [cross | b1b2] (NTT form)
-            for (int i = 0; i < cnt; i++) {
-                const size_t tot = 2 * lq;
-                add_kernel<<<blocks_for(tot, 256), 256, 0, st>>>(dc, out + (size_t)i * 2 * lq, tz + (size_t)i * 3 * lq + lq,
-                                                                 out + (size_t)i * 2 * lq, tot, dc.nq);
-            }
-            check_launch("relin_add");
+            // [cross | b1b2] (NTT form) added at the tail's store
+            ks_tail(dc, m.sd2, d_rlk, dc.dnum, m.se, nullptr, pb, cnt, st, KsExtra{tz + lq, 3 * lq, 0});
         }
     });
 }

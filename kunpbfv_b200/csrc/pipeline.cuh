@@ -331,6 +331,7 @@ struct OutKeyRow {
     size_t ds, ks;
     int ndig;
     uint64_t q, mh, ml, mp, pinv, pinvs;
+    const uint64_t* extra;  // a term in NTT form to add, or null
     // v below 8q
     template <int K>
     __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
@@ -338,8 +339,24 @@ struct OutKeyRow {
         key_product<K>(dig, key, ds, ks, ndig, q, mh, ml, mp, j, ip);
 #pragma unroll
         for (int i = 0; i < K; i++)
-            p[j[i]] = reduce_from(csub63(v[i], q << 2) + shoup4(ip[i], pinv, pinvs, q), q, 3);
+            ip[i] = reduce_from(csub63(v[i], q << 2) + shoup4(ip[i], pinv, pinvs, q), q, 3);
+        if (extra) {
+            uint64_t e[K];
+#pragma unroll
+            for (int i = 0; i < K; i++) e[i] = __ldg(extra + j[i]);
+#pragma unroll
+            for (int i = 0; i < K; i++) ip[i] = add_mod(ip[i], e[i], q);
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++) p[j[i]] = ip[i];
     }
+};
+// NTT-form terms that the key-switch tail adds to the output halves h >= from:
+// base + item * stride + ((h - from) nq + l) N (base null: none)
+struct KsExtra {
+    const uint64_t* base = nullptr;
+    size_t stride = 0;
+    int from = 0;
 };
 struct OutCtKeyDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
     PtrBatch pb;
@@ -347,6 +364,7 @@ struct OutCtKeyDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
     const uint64_t* rlk;  // [ndig][2][Q|P] of the top level
     DevConsts dc;
     int ndig;
+    KsExtra ex;
     __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
     __device__ __forceinline__ OutKeyRow bind(int row) const {
         const int nq = dc.nq, logn = dc.logn;
@@ -360,6 +378,7 @@ struct OutCtKeyDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
         r.ndig = ndig;
         r.q = dc.mods[l]; r.mh = dc.mu_hi[l]; r.ml = dc.mu_lo[l]; r.mp = dc.mu_prod[l];
         r.pinv = dc.pinv_q[l]; r.pinvs = dc.pinv_qs[l];
+        r.extra = ex.base && h >= ex.from ? ex.base + item * ex.stride + (((size_t)(h - ex.from) * nq + l) << logn) : nullptr;
         return r;
     }
 };
@@ -441,7 +460,7 @@ void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* ou
 void lift_launch(const DevConsts& dc, uint64_t* sd2, int count, cudaStream_t st);
 // key-switch tail: key product, mod down and add, written to the outputs of pb
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
-             const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st);
+             const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st, const KsExtra& ex = {});
 // the auxiliary streams and fork / join events of the sub-batches (created once)
 void ensure_branch_streams(Context& c);
 // the whole multiply + relinearise of one sub-batch (9 launches)

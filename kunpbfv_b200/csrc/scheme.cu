@@ -70,39 +70,190 @@ static void sample_uniform(Context& c, const uint8_t seed[32], uint32_t domain, 
     check_launch("sample_uniform");
 }
 
-// ---- pointer-table variants of encryption, decryption and addition ----------
-// delta * m of item i (plaintext pb.a[i]) into its work slot
-__global__ void delta_m_ptr_kernel(DevConsts c, PtrBatch pb, uint64_t* __restrict__ work, size_t total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const size_t lq = (size_t)c.nq << c.logn;
-    const size_t item = i / lq, w = i % lq;
-    const int l = (int)(w >> c.logn);
-    const uint64_t mv = pb.a[item][w & (((size_t)1 << c.logn) - 1)];
-    const uint64_t mq = shoup(mv, c.negq_mod_t, c.negq_mod_t_s, c.t);
-    work[item * 4 * lq + 3 * lq + w] = shoup(mq, c.tinv_q[l], c.tinv_qs[l], c.mods[l]);
+// ---- encryption: ct = [v pk.a + e0 | v pk.b + e1 + delta m] in NTT form
+// (encryptZero / encryptMsg, include/BFVScheme.cuh:87-146) -----------------------
+// Small polynomials stay small: one kernel draws v (ternary), e0 and e1
+// (Gaussian) as bytes and -Q m mod t per coefficient; the forward NTTs' loads turn
+// them into residues of their prime, e1 and delta m entering one transform
+// together; the second one's stores multiply by the public key. Against
+// samplers that wrote every limb, a delta m launch per item, four transforms
+// per limb and a combination kernel, 64 encryptions with encoding at N = 16384, 7
+// primes went from 969 to 423 us.
+struct EncIn {
+    uint64_t id[kMaxBatch];
+    const uint64_t* m[kMaxBatch];
+};
+// item i: small + 3 N i: v, e0, e1; mq + N i: (-Q mod t) m mod t
+__global__ void sample_enc_kernel(DevConsts c, SalsaKey kv, SalsaKey k0, SalsaKey k1, EncIn in, int8_t* __restrict__ small,
+                                  uint64_t* __restrict__ mq, int items) {
+    __shared__ uint64_t cdt[64];
+    const int steps = 2 * c.gauss_bound;  // thresholds, in order
+    if ((int)threadIdx.x < 64) cdt[threadIdx.x] = (int)threadIdx.x < steps ? c.gauss_cdt[threadIdx.x] : UINT64_MAX;
+    __syncthreads();
+    const unsigned n = 1u << c.logn, per = n / 16 + n / 4;  // keystream blocks of one item
+    const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned item = gid / per, r = gid % per;
+    if (item >= (unsigned)items) return;
+    const uint64_t id = in.id[item];
+    uint32_t w[16];
+    int8_t* out = small + (size_t)item * 3 * n;
+    if (r < n / 16) {  // 16 ternary values
+        salsa_block(kv, (uint32_t)id, (uint32_t)(id >> 32), r, w);
+        uint32_t b[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < 16; s++) {
+            const uint32_t u = (uint32_t)(((uint64_t)w[s] * 3) >> 32);
+            b[s / 4] |= (u == 2 ? 255u : u) << (8 * (s & 3));
+        }
+        *reinterpret_cast<uint4*>(out + (size_t)r * 16) = make_uint4(b[0], b[1], b[2], b[3]);
+        return;
+    }
+    const unsigned e = r - n / 16, which = e >= n / 8, blk = which ? e - n / 8 : e;  // 8 Gaussian values
+    salsa_block(which ? k1 : k0, (uint32_t)id, (uint32_t)(id >> 32), blk, w);
+    uint32_t b[2] = {0, 0};
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+        const uint64_t u = (uint64_t)w[2 * s] | ((uint64_t)w[2 * s + 1] << 32);
+        int pos = 0;  // thresholds <= u
+#pragma unroll
+        for (int h = 32; h > 0; h >>= 1)
+            if (pos + h <= steps && u >= cdt[pos + h - 1]) pos += h;
+        b[s / 4] |= (uint32_t)(uint8_t)(int8_t)(pos - c.gauss_bound) << (8 * (s & 3));
+    }
+    *reinterpret_cast<uint2*>(out + (size_t)(1 + which) * n + (size_t)blk * 8) = make_uint2(b[0], b[1]);
+    if (which) {
+        const uint64_t* m = in.m[item] + (size_t)blk * 8;
+        ulonglong2* o = reinterpret_cast<ulonglong2*>(mq + (size_t)item * n + (size_t)blk * 8);
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+            o[s] = make_ulonglong2(shoup(m[2 * s], c.negq_mod_t, c.negq_mod_t_s, c.t),
+                                   shoup(m[2 * s + 1], c.negq_mod_t, c.negq_mod_t_s, c.t));
+    }
 }
-__global__ void enc_combine_ptr_kernel(DevConsts c, const uint64_t* __restrict__ pk, const uint64_t* __restrict__ work,
-                                       PtrBatch pb, size_t total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const size_t lq = (size_t)c.nq << c.logn;
-    const size_t item = i / lq, w = i % lq;
-    const int l = (int)(w >> c.logn);
-    const uint64_t q = c.mods[l], mh = c.mu_hi[l], ml = c.mu_lo[l];
-    const uint64_t* wk = work + item * 4 * lq;
-    const uint64_t v = wk[w], e0 = wk[lq + w], e1 = wk[2 * lq + w], dm = wk[3 * lq + w];
-    uint64_t* ct = pb.o[item];
-    ct[w] = add_mod(mul_mod(v, pk[w], q, mh, ml), e0, q);
-    ct[lq + w] = add_mod(add_mod(mul_mod(v, pk[lq + w], q, mh, ml), e1, q), dm, q);
+// a small polynomial (and delta m = ceil(Q m / t)) as residues of one prime, below 5q
+struct EncSmallRow {
+    const int8_t* e;
+    const uint64_t* mq;  // or null
+    uint64_t q, w, ws;   // 1/t mod q
+    __device__ __forceinline__ uint64_t load(int j) const {
+        const int x = e[j];
+        uint64_t v = x < 0 ? q - (uint64_t)(-x) : (uint64_t)x;
+        if (mq) v += shoup4(mq[j], w, ws, q);
+        return v;
+    }
+    __device__ __forceinline__ void store(int, uint64_t) const {}
+};
+struct EncSrc {  // rows (item, poly of `polys` from `first`, l); poly 2 (e1) takes delta m
+    const int8_t* small;
+    const uint64_t* mq;
+    DevConsts dc;
+    int first, polys;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
+    __device__ __forceinline__ EncSmallRow bind(int row) const {
+        const int per = polys * dc.nq, item = row / per, w = row % per, p = first + w / dc.nq, l = w % dc.nq;
+        return EncSmallRow{small + (((size_t)item * 3 + p) << dc.logn),
+                           p == 2 ? mq + ((size_t)item << dc.logn) : nullptr, dc.mods[l], dc.tinv_q[l], dc.tinv_qs[l]};
+    }
+};
+// output rows (item, h, l): + v pk[h] (NTT form, fully reduced)
+struct EncOutRow {
+    static constexpr bool kStoreMany = true;
+    uint64_t* p;
+    const uint64_t *v, *pk;
+    uint64_t q, mp;
+    template <int K>
+    __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&x)[K]) const {
+        uint64_t a[K], b[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            a[i] = __ldg(v + j[i]);
+            b[i] = __ldg(pk + j[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < K; i++)
+            p[j[i]] = reduce_from(csub63(x[i], q << 2) + barrett_prod_lazy(mul_wide(a[i], b[i]), q, mp), q, 3);
+    }
+};
+struct EncDst {
+    PtrBatch pb;
+    const uint64_t *v, *pk;
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
+    __device__ __forceinline__ EncOutRow bind(int row) const {
+        const int nq = dc.nq, item = row / (2 * nq), w = row % (2 * nq), l = w % nq;
+        return EncOutRow{pb.o[item] + ((size_t)w << dc.logn), v + (((size_t)item * nq + l) << dc.logn),
+                         pk + ((size_t)w << dc.logn), dc.mods[l], dc.mu_prod[l]};
+    }
+};
+static inline OutCtDst plain_of(const EncDst& d) { return OutCtDst{d.pb, d.dc.logn, d.dc.nq}; }
+
+// `cnt` items: plaintexts in.m, ciphertexts pb.o
+static void encrypt_chunk(Context& c, const uint8_t seed[32], const EncIn& in, const PtrBatch& pb, const uint64_t* pk,
+                          int cnt, cudaStream_t st) {
+    const size_t lq = (size_t)c.nq * c.n;
+    uint64_t* v = (uint64_t*)ensure_scratch(c, (size_t)cnt * (lq * 8 + c.n * 8 + 3 * c.n));
+    uint64_t* mq = v + (size_t)cnt * lq;
+    int8_t* small = (int8_t*)(mq + (size_t)cnt * c.n);
+    const size_t blocks = (size_t)cnt * (c.n / 16 + c.n / 4);
+    sample_enc_kernel<<<blocks_for(blocks, 128), 128, 0, st>>>(c.dc, subkey_for(seed, DOM_ENC_V, 0),
+                                                               subkey_for(seed, DOM_ENC_E0, 0),
+                                                               subkey_for(seed, DOM_ENC_E1, 0), in, small, mq, cnt);
+    check_launch("sample_enc");
+    ntt_fwd(c.dc, EncSrc{small, mq, c.dc, 0, 1}, rows_io(c.dc, v, 0, c.nq), cnt * c.nq, st);
+    ntt_fwd(c.dc, EncSrc{small, mq, c.dc, 1, 2}, EncDst{pb, v, pk, c.dc}, cnt * 2 * c.nq, st);
 }
+
+// ---- plaintext addition: b += NTT(delta m) (BFVScheme.cuh:192-217) --------------
+struct DeltaRow {
+    const uint64_t* m;
+    uint64_t a, as, t, w, ws, q;
+    __device__ __forceinline__ uint64_t load(int j) const { return shoup4(shoup(m[j], a, as, t), w, ws, q); }
+    __device__ __forceinline__ void store(int, uint64_t) const {}
+};
+struct DeltaSrc {  // rows (item, l)
+    const uint64_t* m;
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
+    __device__ __forceinline__ DeltaRow bind(int row) const {
+        const int item = row / dc.nq, l = row % dc.nq;
+        return DeltaRow{m + ((size_t)item << dc.logn), dc.negq_mod_t, dc.negq_mod_t_s, dc.t,
+                        dc.tinv_q[l], dc.tinv_qs[l], dc.mods[l]};
+    }
+};
+struct AddPlainRow {
+    static constexpr bool kStoreMany = true;
+    const uint64_t* b;
+    uint64_t* out;  // may be b
+    uint64_t q;
+    template <int K>
+    __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
+        uint64_t x[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) x[i] = b[j[i]];
+#pragma unroll
+        for (int i = 0; i < K; i++) out[j[i]] = add_mod(x[i], reduce_from(v[i], q, 3), q);
+    }
+};
+struct AddPlainDst {  // rows (item, l) of the b parts
+    const uint64_t* ct;
+    uint64_t* out;
+    uint64_t* rows;  // plain rows of a split transform
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
+    __device__ __forceinline__ AddPlainRow bind(int row) const {
+        const int item = row / dc.nq, l = row % dc.nq;
+        const size_t at = (((size_t)item * 2 + 1) * dc.nq + l) << dc.logn;
+        return AddPlainRow{ct + at, out + at, dc.mods[l]};
+    }
+};
+static inline RowsIO plain_of(const AddPlainDst& d) { return RowsIO{d.rows, d.dc.logn, 0, d.dc.nq}; }
+
 // x = pb.a[item], y = pb.b[item], out = pb.o[item]: 2 x nq limbs each; grid.y = item
-__global__ void add_ptr_kernel(DevConsts c, PtrBatch pb, size_t per_item) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= per_item) return;
+__global__ void add_ptr_kernel(DevConsts c, PtrBatch pb) {
+    const RowAt r = row_at<1>(c.logn);
+    const size_t i = ((size_t)r.row << c.logn) + r.j;
     const int item = blockIdx.y;
-    const int l = (int)((i >> c.logn) % c.nq);
-    pb.o[item][i] = add_mod(pb.a[item][i], pb.b[item][i], c.mods[l]);
+    pb.o[item][i] = add_mod(pb.a[item][i], pb.b[item][i], c.mods[r.row % c.nq]);
 }
 // decryption source with ciphertexts at pb.a[item]
 struct DecSrcP {
@@ -244,10 +395,8 @@ int kbfv_encode(kbfv_context* ctx, const uint64_t* d_slots, uint64_t* d_m, uint3
     return guarded([&] {
         Context& c = CX(ctx);
         if (!count) return;
-        if (d_m != d_slots)
-            KB_CHECK_CUDA(cudaMemcpyAsync(d_m, d_slots, (size_t)count * c.n * 8, cudaMemcpyDeviceToDevice, S(stream)));
-        RowsIO io = rows_io(c.dc, d_m, c.dc.idx_pt, 1);
-        ntt_inv(c.dc, io, io, (int)count, S(stream));
+        ntt_inv(c.dc, rows_io(c.dc, const_cast<uint64_t*>(d_slots), c.dc.idx_pt, 1), rows_io(c.dc, d_m, c.dc.idx_pt, 1),
+                (int)count, S(stream));
     });
 }
 
@@ -255,10 +404,8 @@ int kbfv_decode(kbfv_context* ctx, const uint64_t* d_m, uint64_t* d_slots, uint3
     return guarded([&] {
         Context& c = CX(ctx);
         if (!count) return;
-        if (d_m != d_slots)
-            KB_CHECK_CUDA(cudaMemcpyAsync(d_slots, d_m, (size_t)count * c.n * 8, cudaMemcpyDeviceToDevice, S(stream)));
-        RowsIO io = rows_io(c.dc, d_slots, c.dc.idx_pt, 1);
-        ntt_fwd(c.dc, io, io, (int)count, S(stream));
+        ntt_fwd(c.dc, rows_io(c.dc, const_cast<uint64_t*>(d_m), c.dc.idx_pt, 1), rows_io(c.dc, d_slots, c.dc.idx_pt, 1),
+                (int)count, S(stream));
     });
 }
 
@@ -294,23 +441,14 @@ int kbfv_encrypt(kbfv_context* ctx, const uint8_t seed[32], uint64_t enc_id, con
         const size_t lq = (size_t)c.nq * c.n;
         for (uint32_t off = 0; off < count; off += kMaxBatch) {
             const int cnt = (int)std::min<uint32_t>(kMaxBatch, count - off);
-            uint64_t* work = (uint64_t*)ensure_scratch(c, (size_t)cnt * 4 * lq * 8);
-            const uint64_t id0 = enc_id + off;
-            // [v | e0 | e1 | dm] per item
-            sample_small(c, seed, DOM_ENC_V, id0, 0, 0, c.nq, work, 4 * lq, cnt, st);
-            sample_small(c, seed, DOM_ENC_E0, id0, 1, 0, c.nq, work + lq, 4 * lq, cnt, st);
-            sample_small(c, seed, DOM_ENC_E1, id0, 1, 0, c.nq, work + 2 * lq, 4 * lq, cnt, st);
+            EncIn in{};
+            PtrBatch pb{};
             for (int i = 0; i < cnt; i++) {
-                const size_t tot = lq;
-                delta_m_kernel<<<blocks_for(tot, 256), 256, 0, st>>>(c.dc, d_m + (size_t)(off + i) * c.n,
-                                                                      work + (size_t)i * 4 * lq + 3 * lq, tot);
+                in.id[i] = enc_id + off + i;
+                in.m[i] = d_m + (size_t)(off + i) * c.n;
+                pb.o[i] = d_ct + (size_t)(off + i) * 2 * lq;
             }
-            check_launch("delta_m");
-            RowsIO io = rows_io(c.dc, work, 0, c.nq);
-            ntt_fwd(c.dc, io, io, cnt * 4 * c.nq, st);
-            const size_t total = (size_t)cnt * lq;
-            enc_combine_kernel<<<stride_blocks(total, 256), 256, 0, st>>>(c.dc, d_pk, work, d_ct + (size_t)off * 2 * lq, total);
-            check_launch("enc_combine");
+            encrypt_chunk(c, seed, in, pb, d_pk, cnt, st);
         }
     });
 }
@@ -340,10 +478,9 @@ int kbfv_add(kbfv_context* ctx, const uint64_t* d_x, const uint64_t* d_y, uint64
              kbfv_stream stream) {
     return guarded([&] {
         Context& c = CX(ctx);
-        const size_t total = (size_t)count * 2 * c.nq * c.n;
-        if (!total) return;
-        add_kernel<<<blocks_for(total, 256), 256, 0, S(stream)>>>(c.dc, d_x, d_y, d_out, total, c.nq);
-        check_launch("add");
+        if (!count) return;
+        const size_t per = (size_t)2 * c.nq * c.n;
+        launch_add(c.dc, d_x, per, d_y, per, d_out, per, count, 2 * c.nq, c.nq, S(stream));
     });
 }
 
@@ -351,9 +488,12 @@ int kbfv_mul_plain(kbfv_context* ctx, const uint64_t* d_ct, const uint64_t* d_pt
                    kbfv_stream stream) {
     return guarded([&] {
         Context& c = CX(ctx);
-        const size_t total = (size_t)count * 2 * c.nq * c.n;
-        if (!total) return;
-        mul_plain_kernel<<<blocks_for(total, 256), 256, 0, S(stream)>>>(c.dc, d_ct, d_pt_ntt, d_out, total);
+        const size_t rows = (size_t)count * 2 * c.nq;
+        if (!rows) return;
+        if (aligned16({d_ct, d_pt_ntt, d_out}))
+            mul_plain_kernel<2><<<row_blocks<2>(rows, c.logn), 256, 0, S(stream)>>>(c.dc, d_ct, d_pt_ntt, d_out);
+        else
+            mul_plain_kernel<1><<<row_blocks<1>(rows, c.logn), 256, 0, S(stream)>>>(c.dc, d_ct, d_pt_ntt, d_out);
         check_launch("mul_plain");
     });
 }
@@ -368,20 +508,13 @@ int kbfv_add_plain(kbfv_context* ctx, const uint64_t* d_ct, const uint64_t* d_m,
         const size_t lq = (size_t)c.nq * c.n;
         for (uint32_t off = 0; off < count; off += kMaxBatch) {
             const int cnt = (int)std::min<uint32_t>(kMaxBatch, count - off);
-            uint64_t* dm = (uint64_t*)ensure_scratch(c, (size_t)cnt * lq * 8);
-            delta_m_kernel<<<blocks_for((size_t)cnt * lq, 256), 256, 0, st>>>(c.dc, d_m + (size_t)off * c.n, dm,
-                                                                             (size_t)cnt * lq);
-            check_launch("delta_m");
-            RowsIO io = rows_io(c.dc, dm, 0, c.nq);
-            ntt_fwd(c.dc, io, io, cnt * c.nq, st);
-            for (int i = 0; i < cnt; i++) {
-                const uint64_t* src = d_ct + (size_t)(off + i) * 2 * lq;
-                uint64_t* dst = d_out + (size_t)(off + i) * 2 * lq;
-                if (dst != src) KB_CHECK_CUDA(cudaMemcpyAsync(dst, src, lq * 8, cudaMemcpyDeviceToDevice, st));
-                add_kernel<<<blocks_for(lq, 256), 256, 0, st>>>(c.dc, src + lq, dm + (size_t)i * lq, dst + lq, lq,
-                                                                c.nq);
-            }
-            check_launch("add_plain");
+            const uint64_t* src = d_ct + (size_t)off * 2 * lq;
+            uint64_t* dst = d_out + (size_t)off * 2 * lq;
+            uint64_t* rows = (uint64_t*)ensure_scratch(c, (size_t)cnt * lq * 8);
+            ntt_fwd(c.dc, DeltaSrc{d_m + (size_t)off * c.n, c.dc}, AddPlainDst{src, dst, rows, c.dc}, cnt * c.nq, st);
+            if (dst != src)  // the a parts
+                KB_CHECK_CUDA(cudaMemcpy2DAsync(dst, 2 * lq * 8, src, 2 * lq * 8, lq * 8, (size_t)cnt,
+                                                cudaMemcpyDeviceToDevice, st));
         }
     });
 }
@@ -433,14 +566,17 @@ static int linear_op(kbfv_context* ctx, const uint64_t* x, const uint64_t* y, ui
     return guarded([&] {
         Context& c = CX(ctx);
         KB_REQUIRE(x && out && (op == 1 || op == 2 || y), KBFV_ERR_INVALID, "null argument");
-        const size_t total = (size_t)count * 2 * c.nq * c.n;
-        if (!total) return;
+        const size_t rows = (size_t)count * 2 * c.nq;
+        if (!rows) return;
         ScalarTab tab{};
         for (int l = 0; op >= 2 && l < c.nq; l++) {
             tab.c[l] = cnst % c.mods[l];
             tab.cs[l] = H::shoup(tab.c[l], c.mods[l]);
         }
-        linear_kernel<<<blocks_for(total, 256), 256, 0, S(stream)>>>(c.dc, x, y, out, total, c.nq, op, tab);
+        if (aligned16({x, y, out}))
+            linear_kernel<2><<<row_blocks<2>(rows, c.logn), 256, 0, S(stream)>>>(c.dc, x, y, out, c.nq, op, tab);
+        else
+            linear_kernel<1><<<row_blocks<1>(rows, c.logn), 256, 0, S(stream)>>>(c.dc, x, y, out, c.nq, op, tab);
         check_launch("linear");
     });
 }
@@ -502,27 +638,16 @@ int kbfv_encrypt_batch(kbfv_context* ctx, const uint8_t seed[32], const uint64_t
         if (!seed) seed = c.seed;
         KB_REQUIRE(enc_ids && d_pk && d_m && d_ct, KBFV_ERR_INVALID, "null argument");
         cudaStream_t st = S(stream);
-        const size_t lq = (size_t)c.nq * c.n;
         for (uint32_t off = 0; off < count; off += kMaxBatch) {
             const int cnt = (int)std::min<uint32_t>(kMaxBatch, count - off);
-            PtrBatch pb = make_batch(d_m + off, d_m + off, d_ct + off, cnt);
-            IdTable ids{};
-            for (int i = 0; i < cnt; i++) ids.v[i] = enc_ids[off + i];
-            uint64_t* work = (uint64_t*)ensure_scratch(c, (size_t)cnt * 4 * lq * 8);
-            const size_t per = c.n / 16, per8 = c.n / 8;
-            const SalsaKey kv = subkey_for(seed, DOM_ENC_V, 0), k0 = subkey_for(seed, DOM_ENC_E0, 0),
-                           k1 = subkey_for(seed, DOM_ENC_E1, 0);
-            sample_small_ids_kernel<0><<<blocks_for(per * cnt, 128), 128, 0, st>>>(c.dc, kv, ids, 0, c.nq, work, 4 * lq, cnt);
-            sample_small_ids_kernel<1><<<blocks_for(per8 * cnt, 128), 128, 0, st>>>(c.dc, k0, ids, 0, c.nq, work + lq, 4 * lq, cnt);
-            sample_small_ids_kernel<1><<<blocks_for(per8 * cnt, 128), 128, 0, st>>>(c.dc, k1, ids, 0, c.nq, work + 2 * lq, 4 * lq, cnt);
-            check_launch("sample_small");
-            const size_t total = (size_t)cnt * lq;
-            delta_m_ptr_kernel<<<stride_blocks(total, 256), 256, 0, st>>>(c.dc, pb, work, total);
-            check_launch("delta_m");
-            RowsIO io = rows_io(c.dc, work, 0, c.nq);
-            ntt_fwd(c.dc, io, io, cnt * 4 * c.nq, st);
-            enc_combine_ptr_kernel<<<stride_blocks(total, 256), 256, 0, st>>>(c.dc, d_pk, work, pb, total);
-            check_launch("enc_combine");
+            EncIn in{};
+            PtrBatch pb{};
+            for (int i = 0; i < cnt; i++) {
+                in.id[i] = enc_ids[off + i];
+                in.m[i] = d_m[off + i];
+                pb.o[i] = d_ct[off + i];
+            }
+            encrypt_chunk(c, seed, in, pb, d_pk, cnt, st);
         }
     });
 }
@@ -554,11 +679,10 @@ int kbfv_add_batch(kbfv_context* ctx, const uint64_t* const* d_x, const uint64_t
     return guarded([&] {
         Context& c = CX(ctx);
         KB_REQUIRE(d_x && d_y && d_out, KBFV_ERR_INVALID, "null argument");
-        const size_t per = (size_t)2 * c.nq * c.n;
         for (uint32_t off = 0; off < count; off += kMaxBatch) {
             const int cnt = (int)std::min<uint32_t>(kMaxBatch, count - off);
             PtrBatch pb = make_batch(d_x + off, d_y + off, d_out + off, cnt);
-            add_ptr_kernel<<<dim3(blocks_for(per, 256), (unsigned)cnt), 256, 0, S(stream)>>>(c.dc, pb, per);
+            add_ptr_kernel<<<dim3(row_blocks<1>(2 * c.nq, c.logn), (unsigned)cnt), 256, 0, S(stream)>>>(c.dc, pb);
             check_launch("add_batch");
         }
     });
