@@ -188,7 +188,10 @@ void build_context(Context& c, const kbfv_params& prm) {
     DevConsts& dc = c.dc;
     // two coefficients per base-conversion thread: 16% fewer IMAD instructions,
     // 8% faster than one at N=16384, 7 + 1 primes, 32-pair sub-batches (B200)
-    dc.shape = LaunchShape{kSplitRows14Default, 256, 2, 128, 2, 1, 1, kSplitRowsAloneDefault};
+    int sms = 0, dev = 0;
+    KB_CHECK_CUDA(cudaGetDevice(&dev));
+    KB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    dc.shape = LaunchShape{kSplitRows14Default, 256, 2, 128, 2, 1, 1, kSplitRowsAloneDefault, sms};
     dc.logn = c.logn; dc.nq = c.nq; dc.np = c.np; dc.nr = c.nr; dc.nt = c.nt;
     dc.dnum = c.dnum; dc.alpha = c.alpha; dc.npq = c.nq + c.np; dc.nqr = c.nq + c.nr;
     dc.idx_p = c.nq; dc.idx_r = c.nq + c.np; dc.idx_t = c.nq + c.np + c.nr; dc.idx_pt = nall - 1;

@@ -27,6 +27,7 @@ struct LaunchShape {
                          // loader of the NTT over R (no K2 launch)
     int l2_prefetch;     // 1: block kernels ask L2 for the block one wave of CTAs ahead
     int split_rows_alone;  // split_rows14 for a multiply that runs as one stream
+    int tail_sms;        // SMs whose last wave of N = 2^14 transforms may run split (split14); 0: beside a sibling sub-batch
 };
 
 // Everything a kernel needs, passed by value (all pointers into one device pool).

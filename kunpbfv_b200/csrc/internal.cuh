@@ -165,6 +165,20 @@ constexpr int kSplitRows14Default = 48;
 // default of LaunchShape::split_rows_alone (KBFV_TUNE_SPLIT_ROWS_ALONE).
 constexpr int kSplitRowsAloneDefault = 148;
 
+// Whether `rows` transforms of 2^14 points run split. A wave of whole-ring CTAs
+// (one per SM) takes 25 us however few rows it has; the split form takes 12 us plus
+// 0.19 us a row. So up to five waves, a launch that has the GPU to itself runs
+// split while its last wave holds at most 96 - 14 (waves - 1) rows (150 rows: 53
+// us whole, 41 split; 231: 55, 54; 333: 80, 68; 448: 105, 94; 600: 132, 123; but
+// 296: 56, 64 and 370: 80, 76 not split). Beside a sibling sub-batch the last
+// wave's idle SMs are not idle (tail_sms 0).
+static inline bool split14(const LaunchShape& sh, int rows) {
+    if (rows <= sh.split_rows14) return true;
+    if (sh.tail_sms <= 0) return false;
+    const int waves = (rows + sh.tail_sms - 1) / sh.tail_sms;
+    return waves >= 2 && waves <= 5 && rows - (waves - 1) * sh.tail_sms <= 96 - 14 * (waves - 1);
+}
+
 // Forward NTT of `rows` rows read through `s` and written through `d`.
 // For logn <= 14 one block kernel (N = 2^14 with at most shape.split_rows14 rows:
 // as for 15/16 with a radix-4 column pass); for 15/16 a radix-8/16 column pass
@@ -181,7 +195,7 @@ static void ntt_fwd(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st
         case 12: launch_fwd_block<12, Src, Dst, FULL>(dc, s, d, rows, 12, st); break;
         case 13: launch_fwd_block<13, Src, Dst, FULL>(dc, s, d, rows, 13, st); break;
         case 14: {
-            if (rows > dc.shape.split_rows14) {
+            if (!split14(dc.shape, rows)) {
                 launch_fwd_block<14, Src, Dst, FULL>(dc, s, d, rows, 14, st);
                 break;
             }
@@ -222,7 +236,7 @@ static void ntt_inv(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st
         case 12: launch_inv_block<12, Src, Dst, true>(dc, s, d, rows, 12, st); break;
         case 13: launch_inv_block<13, Src, Dst, true>(dc, s, d, rows, 13, st); break;
         case 14: {
-            if (rows > dc.shape.split_rows14) {
+            if (!split14(dc.shape, rows)) {
                 launch_inv_block<14, Src, Dst, true>(dc, s, d, rows, 14, st);
                 break;
             }

@@ -162,8 +162,8 @@ static StageRows stage_rows(const Groups& G, F per, int* total) {
 // G describes) as one launch sequence: the stages of mul_relin_chunk, each over
 // all items, every row with its own level's constants.
 static void mul_relin_mixed(Context& top, const uint64_t* rlk, const PtrBatch& pb, const Groups& G, int count,
-                            const MulScratch& m, cudaStream_t st) {
-    const DevConsts& dc = top.dc;  // ring degree and launch shapes; rows take their level's tables
+                            bool sibling, const MulScratch& m, cudaStream_t st) {
+    const DevConsts dc = sibling ? sibling_consts(top) : top.dc;  // ring degree and launch shapes; rows take their level's tables
     int n = 0;
     // K1: INTT over Q of [a1, b1, a2, b2]
     const StageRows r1 = stage_rows(G, [&](int g) { return 4 * G.nq[g]; }, &n);
@@ -328,7 +328,7 @@ int kbfv_mul_relin_levels(kbfv_context* ctx, const uint64_t* d_rlk, const uint32
                 }
                 G.first[G.ng] = n;
                 if (n == 0) continue;
-                mul_relin_mixed(c, d_rlk, pb, G, n, mul_scratch_layout(c, n, base + (size_t)k * region),
+                mul_relin_mixed(c, d_rlk, pb, G, n, nb > 1, mul_scratch_layout(c, n, base + (size_t)k * region),
                                 k == 0 ? st : c.aux[k - 1]);
             }
             for (int k = 1; k < nb; k++) {

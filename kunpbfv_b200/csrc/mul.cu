@@ -160,7 +160,7 @@ int kbfv_mul_relin_batch(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_
                 if (n <= 0) break;
                 PtrBatch pb = make_batch(ct_a + off + lo, ct_b + off + lo, out + off + lo, n);
                 MulScratch m = mul_scratch_layout(c, n, base + b * each);
-                mul_relin_chunk(c.dc, d_rlk, pb, n, m, b == 0 ? st : c.aux[b - 1]);
+                mul_relin_chunk(sibling_consts(c), d_rlk, pb, n, m, b == 0 ? st : c.aux[b - 1]);
             }
             for (int b = 1; b < nb; b++) {
                 KB_CHECK_CUDA(cudaEventRecord(c.join_ev[b - 1], c.aux[b - 1]));
@@ -292,7 +292,7 @@ int kbfv_mul_relin_host(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_t
             }
             PtrBatch pb = make_batch(A.data(), B.data(), O.data(), n);
             MulScratch m = mul_scratch_layout(c, n, base + k * region);
-            mul_relin_chunk(c.dc, d_rlk, pb, n, m, comp);
+            mul_relin_chunk(sibling_consts(c), d_rlk, pb, n, m, comp);
             KB_CHECK_CUDA(cudaEventRecord(c.hcomp[s], comp));
             if (j >= 1) copy_out(j - 1);
         }

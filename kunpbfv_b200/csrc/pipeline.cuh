@@ -466,6 +466,12 @@ void ensure_branch_streams(Context& c);
 // the whole multiply + relinearise of one sub-batch (9 launches)
 void mul_relin_chunk(const DevConsts& dc, const uint64_t* rlk, const PtrBatch& pb, int count, const MulScratch& m,
                      cudaStream_t st);
+// the constants of a sub-batch beside another on a sibling stream
+static inline DevConsts sibling_consts(const Context& c) {
+    DevConsts d = c.dc;
+    d.shape.tail_sms = 0;
+    return d;
+}
 // The constants with the launch shapes of a multiply that runs as one stream
 // (no sibling sub-batch on another stream to fill the SMs): 2^14-point
 // transforms of up to shape.split_rows_alone rows run split.
