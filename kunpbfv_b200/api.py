@@ -371,6 +371,11 @@ class BFVContext:
         torch = _torch()
         return torch.zeros(shape, dtype=torch.int64, device="cuda")
 
+    def empty(self, *shape):
+        """an output buffer that the call writes whole (no fill launch over it first)"""
+        torch = _torch()
+        return torch.empty(shape, dtype=torch.int64, device="cuda")
+
     @classmethod
     def from_bits(cls, log_n: int, q_bits, p_bits, plain_modulus: int, dnum: int = 1) -> "BFVContext":
         """Parameter set from per-prime bit sizes (kbfv_params_create), e.g.
@@ -418,19 +423,19 @@ class BFVContext:
     # ---- encoder (include/Encoder.cuh)
     def encode(self, slots, out=None, stream=None):
         count = slots.numel() // self.N
-        out = out if out is not None else self.zeros(count, self.N)
+        out = out if out is not None else self.empty(count, self.N)
         _check(lib().kbfv_encode(self._h, _ptr(slots), _ptr(out), count, _stream_ptr(stream)))
         return out
 
     def decode(self, m, out=None, stream=None):
         count = m.numel() // self.N
-        out = out if out is not None else self.zeros(count, self.N)
+        out = out if out is not None else self.empty(count, self.N)
         _check(lib().kbfv_decode(self._h, _ptr(m), _ptr(out), count, _stream_ptr(stream)))
         return out
 
     def encode_ntt(self, vals, out=None, stream=None):
         count = vals.numel() // self.N
-        out = out if out is not None else self.zeros(count, self.q_count, self.N)
+        out = out if out is not None else self.empty(count, self.q_count, self.N)
         _check(lib().kbfv_encode_ntt(self._h, _ptr(vals), _ptr(out), count, _stream_ptr(stream)))
         return out
 
@@ -442,38 +447,38 @@ class BFVContext:
 
     def bconv_q_to_r(self, x, stream=None):
         polys = x.numel() // (self.q_count * self.N)
-        return self._op("kbfv_bconv_q_to_r", [x], self.zeros(polys, self.r_count, self.N), polys, stream)
+        return self._op("kbfv_bconv_q_to_r", [x], self.empty(polys, self.r_count, self.N), polys, stream)
 
     def bconv_r_to_q(self, x, stream=None):
         polys = x.numel() // (self.r_count * self.N)
-        return self._op("kbfv_bconv_r_to_q", [x], self.zeros(polys, self.q_count, self.N), polys, stream)
+        return self._op("kbfv_bconv_r_to_q", [x], self.empty(polys, self.q_count, self.N), polys, stream)
 
     def tensor_qr(self, c1, c2, stream=None):
         nqr = self.q_count + self.r_count
         pairs = c1.numel() // (2 * nqr * self.N)
-        return self._op("kbfv_tensor_qr", [c1, c2], self.zeros(pairs, 3, nqr, self.N), pairs, stream)
+        return self._op("kbfv_tensor_qr", [c1, c2], self.empty(pairs, 3, nqr, self.N), pairs, stream)
 
     def scale_round_qr_r(self, x, stream=None):
         polys = x.numel() // ((self.q_count + self.r_count) * self.N)
-        return self._op("kbfv_scale_round_qr_r", [x], self.zeros(polys, self.r_count, self.N), polys, stream)
+        return self._op("kbfv_scale_round_qr_r", [x], self.empty(polys, self.r_count, self.N), polys, stream)
 
     def decrypt_round(self, x, stream=None):
         polys = x.numel() // (self.q_count * self.N)
-        return self._op("kbfv_decrypt_round", [x], self.zeros(polys, self.N), polys, stream)
+        return self._op("kbfv_decrypt_round", [x], self.empty(polys, self.N), polys, stream)
 
     def delta_m(self, m, stream=None):
         polys = m.numel() // self.N
-        return self._op("kbfv_delta_m", [m], self.zeros(polys, self.q_count, self.N), polys, stream)
+        return self._op("kbfv_delta_m", [m], self.empty(polys, self.q_count, self.N), polys, stream)
 
     def modup(self, x, stream=None):
         polys = x.numel() // (self.q_count * self.N)
         npq = self.q_count + self.p_count
-        return self._op("kbfv_modup", [x], self.zeros(polys, self.dnum, npq, self.N), polys, stream)
+        return self._op("kbfv_modup", [x], self.empty(polys, self.dnum, npq, self.N), polys, stream)
 
     def moddown(self, x, stream=None):
         npq = self.q_count + self.p_count
         polys = x.numel() // (npq * self.N)
-        return self._op("kbfv_moddown", [x], self.zeros(polys, self.q_count, self.N), polys, stream)
+        return self._op("kbfv_moddown", [x], self.empty(polys, self.q_count, self.N), polys, stream)
 
     # ---- key switch over the T base (the reference's KLSS)
     def klss_info(self):
@@ -485,17 +490,17 @@ class BFVContext:
     def klss_modup_qj_to_t(self, x, stream=None):
         _, nqj, _ = self.klss_info()
         polys = x.numel() // (self.q_count * self.N)
-        return self._op("kbfv_klss_modup_qj_to_t", [x], self.zeros(polys, nqj, self.t_count, self.N), polys, stream)
+        return self._op("kbfv_klss_modup_qj_to_t", [x], self.empty(polys, nqj, self.t_count, self.N), polys, stream)
 
     def klss_modup_pq_to_t(self, x, stream=None):
         nri, _, _ = self.klss_info()
         polys = x.numel() // ((self.q_count + self.p_count) * self.N)
-        return self._op("kbfv_klss_modup_pq_to_t", [x], self.zeros(polys, nri, self.t_count, self.N), polys, stream)
+        return self._op("kbfv_klss_modup_pq_to_t", [x], self.empty(polys, nri, self.t_count, self.N), polys, stream)
 
     def klss_external_product(self, digits, key_t, stream=None):
         nri, nqj, _ = self.klss_info()
         count = digits.numel() // (nqj * self.t_count * self.N)
-        out = self.zeros(count, 2, nri, self.t_count, self.N)
+        out = self.empty(count, 2, nri, self.t_count, self.N)
         _check(lib().kbfv_klss_external_product(self._h, _ptr(digits), _ptr(key_t), _ptr(out), count,
                                                 _stream_ptr(stream)))
         return out
@@ -504,7 +509,7 @@ class BFVContext:
         nri, _, _ = self.klss_info()
         polys = x.numel() // (nri * self.t_count * self.N)
         npq = self.q_count + self.p_count
-        return self._op("kbfv_klss_t_to_pq", [x], self.zeros(polys, npq, self.N), polys, stream)
+        return self._op("kbfv_klss_t_to_pq", [x], self.empty(polys, npq, self.N), polys, stream)
 
 
 def reference_context(log_n: int) -> BFVContext:
@@ -554,6 +559,11 @@ class Ciphertext:
     @property
     def bx_device(self):
         return self.cipher_device.view(self.count, 2, self.ctx.q_count, self.ctx.N)[:, 1]
+
+
+def _ciphertext(ctx: BFVContext, count: int) -> Ciphertext:
+    """a ciphertext batch for a call to write"""
+    return Ciphertext(ctx, ctx.empty(count, 2, ctx.q_count, ctx.N))
 
 
 class Tensor3:
@@ -674,20 +684,20 @@ class BFVScheme:
         if enc_id is None:
             enc_id = self._enc_counter
             self._enc_counter += cnt
-        ct = Ciphertext(ctx, count=cnt)
+        ct = _ciphertext(ctx, cnt)
         _check(lib().kbfv_encrypt(ctx.handle, _u8(self.seed), enc_id, _ptr(self.publicKey), _ptr(pt.mx_device),
                                   _ptr(ct.cipher_device), cnt, _stream_ptr(stream)))
         return ct
 
     def decryptMsg(self, sk: SecretKey, ct: Ciphertext, stream=None) -> Plaintext:
         ctx = ct.ctx  # the ciphertext's level
-        pt = Plaintext(ctx, count=ct.count)
+        pt = Plaintext(ctx, ctx.empty(ct.count, ctx.N))
         _check(lib().kbfv_decrypt(ctx.handle, _ptr(sk.sx_device), _ptr(ct.cipher_device), _ptr(pt.mx_device),
                                   ct.count, _stream_ptr(stream)))
         return pt
 
     def add(self, c1: Ciphertext, c2: Ciphertext, stream=None) -> Ciphertext:
-        out = Ciphertext(c1.ctx, count=c1.count)
+        out = _ciphertext(c1.ctx, c1.count)
         _check(lib().kbfv_add(c1.ctx.handle, _ptr(c1.cipher_device), _ptr(c2.cipher_device),
                               _ptr(out.cipher_device), c1.count, _stream_ptr(stream)))
         return out
@@ -697,7 +707,7 @@ class BFVScheme:
                               _ptr(c1.cipher_device), c1.count, _stream_ptr(stream)))
 
     def sub(self, c1: Ciphertext, c2: Ciphertext, stream=None) -> Ciphertext:
-        out = Ciphertext(c1.ctx, count=c1.count)
+        out = _ciphertext(c1.ctx, c1.count)
         _check(lib().kbfv_sub(c1.ctx.handle, _ptr(c1.cipher_device), _ptr(c2.cipher_device), _ptr(out.cipher_device),
                               c1.count, _stream_ptr(stream)))
         return out
@@ -734,7 +744,7 @@ class BFVScheme:
                                     _ptr(ct.cipher_device), ct.count, _stream_ptr(stream)))
 
     def mult(self, c1: Ciphertext, c2: Ciphertext, stream=None) -> Tensor3:
-        out = Tensor3(c1.ctx, count=c1.count)
+        out = Tensor3(c1.ctx, c1.ctx.empty(c1.count, 3, c1.ctx.q_count, c1.ctx.N))
         _check(lib().kbfv_mul(c1.ctx.handle, _ptr(c1.cipher_device), _ptr(c2.cipher_device), _ptr(out.data),
                               c1.count, _stream_ptr(stream)))
         return out
@@ -743,7 +753,7 @@ class BFVScheme:
         if self.rlk is None:
             raise KbfvError(-5, "rotKey_23 not exists")
         cnt = t3.data.numel() // (3 * t3.ctx.q_count * t3.ctx.N)
-        out = Ciphertext(t3.ctx, count=cnt)
+        out = _ciphertext(t3.ctx, cnt)
         if self.relin == "gadget":
             _check(lib().kbfv_relinearize_gadget(t3.ctx.handle, _ptr(self.gk), self.gadget_log_base, _ptr(t3.data),
                                                  _ptr(out.cipher_device), cnt, _stream_ptr(stream)))
@@ -759,7 +769,7 @@ class BFVScheme:
         """Batched ct1[i] * ct2[i] with relinearisation (multAndEqual_23 without the shortcut)."""
         if self.rlk is None:
             raise KbfvError(-5, "rotKey_23 not exists")
-        out = out if out is not None else Ciphertext(c1.ctx, count=c1.count)
+        out = out if out is not None else _ciphertext(c1.ctx, c1.count)
         if self.relin == "gadget":
             _check(lib().kbfv_mul_relin_gadget(c1.ctx.handle, _ptr(self.gk), self.gadget_log_base,
                                                _ptr(c1.cipher_device), _ptr(c2.cipher_device), _ptr(out.cipher_device),
@@ -869,7 +879,7 @@ class BFVScheme:
     def apply_galois(self, ct: Ciphertext, g: int, out: Optional[Ciphertext] = None, stream=None) -> Ciphertext:
         if g not in self.galois_keys:
             raise KbfvError(-5, "rotKey_23 not exists")
-        out = out if out is not None else Ciphertext(ct.ctx, count=ct.count)
+        out = out if out is not None else _ciphertext(ct.ctx, ct.count)
         _check(lib().kbfv_apply_galois(ct.ctx.handle, _ptr(self.galois_keys[g]), g, _ptr(ct.cipher_device),
                                        _ptr(out.cipher_device), ct.count, _stream_ptr(stream)))
         return out
@@ -888,7 +898,7 @@ class BFVScheme:
         """drop the last live prime (divide and round); the result lives at ct.ctx's level - 1"""
         top = ct.ctx._owner or ct.ctx
         lower = top.at_level(ct.ctx.q_count - 1)
-        out = Ciphertext(lower, count=ct.count)
+        out = _ciphertext(lower, ct.count)
         _check(lib().kbfv_mod_switch(ct.ctx.handle, _ptr(ct.cipher_device), _ptr(out.cipher_device), ct.count,
                                      _stream_ptr(stream)))
         return out
@@ -904,7 +914,7 @@ class BFVScheme:
         the output ciphertexts (each at its pair's level)"""
         n = len(pairs)
         if outs is None:
-            outs = [Ciphertext(a.ctx, count=1) for a, _ in pairs]
+            outs = [_ciphertext(a.ctx, 1) for a, _ in pairs]
         lv = (C.c_uint32 * n)(*[a.ctx.q_count for a, _ in pairs])
         A = (VP * n)(*[_ptr(a.cipher_device) for a, _ in pairs])
         B = (VP * n)(*[_ptr(b.cipher_device) for _, b in pairs])
