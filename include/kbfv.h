@@ -283,12 +283,9 @@ typedef enum {
                                     conversions kbfv_bconv_* (2: 16-byte accesses and byte matrix
                                     products on the tensor cores, as in the multiply; 1, and pointers
                                     that are only 8-byte aligned: 64-bit multiply-accumulates) */
-    KBFV_TUNE_FUSE_Q2R_PAIRS = 8, /* 0..128 (default 1): multiplies of at most this many pairs (per
-                                    sub-batch) run the Q -> R base extension in the loader of the
-                                    forward NTT over R: the inverse NTT over Q stores its outputs
-                                    scaled by (Q/q_i)^-1, and there is no base-conversion launch
-                                    and no HBM round trip of the R limbs; each R row then reads
-                                    all q_count Q limbs, which larger batches pay for in L2 traffic */
+    KBFV_TUNE_FUSE_Q2R_PAIRS = 8, /* 0..128 (default 1): accepted, without effect. It chose the batches
+                                    whose Q -> R base extension ran in the loader of the forward
+                                    NTT over R; as a launch of its own it is faster at every size */
     KBFV_TUNE_L2_PREFETCH = 9,   /* 0 or 1 (default): NTT block kernels whose input is plain rows
                                     (standalone transforms, the multiply's INTT of its inputs and
                                     its NTTs over R and Q|P) ask L2 for the block one wave of CTAs

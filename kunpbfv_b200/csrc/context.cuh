@@ -23,8 +23,7 @@ struct LaunchShape {
     int bconv_cpt;       // coefficients per thread of the base conversion (1 or 2)
     int k5_threads;      // CTA size of K5
     int k5_fused_pairs;  // batches of at most this many pairs run K5 as one kernel
-    int fuse_q2r_pairs;  // batches of at most this many pairs run the Q -> R base extension in the
-                         // loader of the NTT over R (no K2 launch)
+    int fuse_q2r_pairs;  // accepted and kept; the base extension is a launch of its own at every size
     int l2_prefetch;     // 1: block kernels ask L2 for the block one wave of CTAs ahead
     int split_rows_alone;  // split_rows14 for a multiply that runs as one stream
     int tail_sms;        // SMs whose last wave of N = 2^14 transforms may run split (split14); 0: beside a sibling sub-batch

@@ -1,10 +1,14 @@
 // The per-coefficient stages of the multiply pipeline as byte matrix products
 // (limb_mma.cuh): K2 (base extension Q -> R), K5 (t/Q scale-and-round Q|R -> R
 // and the base extension R -> Q, chained in registers) and the key-switch
-// digit lift; and K3 with the Q -> R base extension in its loader
-// (q2r_ntt.cuh). Each size of the prime count is instantiated in its own
+// digit lift. Each size of the prime count is instantiated in its own
 // translation unit (k5_m<MAXQ>.cu) so that the unrolled variants compile in
 // parallel.
+//
+// K2 is a launch of its own at every size. Inside the loader of the NTT over R
+// (each row reading all nq words of its coefficients) it saved a launch, but with
+// K2 at 5 us for one pair the fused form was the slower one everywhere: one
+// captured pair 106 -> 111 us at N = 16384, 84 -> 100 at 4096, 292 -> 357 at 32768.
 //
 // A warp takes MT tiles of 16 coefficients of one polynomial per iteration: lane
 // (g = lane / 4, c = lane % 4) coefficients 2g and 2g + 1 of each, the words and
@@ -16,7 +20,6 @@
 #pragma once
 #include "limb_mma.cuh"
 #include "mixed.cuh"
-#include "q2r_ntt.cuh"
 
 // Tiles per iteration: two share one load of the constants as long as their
 // words and sums fit the registers of at least 16 warps per SM.

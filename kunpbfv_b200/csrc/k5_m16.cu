@@ -1,7 +1,6 @@
-// K2, K5 and the fused K3 for contexts of 8 to 15 ciphertext primes
+// K2 and K5 for contexts of 8 to 15 ciphertext primes
 #include "k5_kernels.cuh"
 
-template void q2r_ntt_launch_m<16>(const DevConsts&, const uint64_t*, uint64_t*, int, cudaStream_t);
 template void k2_launch_m<4>(const DevConsts&, const uint64_t*, uint64_t*, int, cudaStream_t);
 template void bconv_mma_launch_m<4>(const DevConsts&, bool, const uint64_t*, uint64_t*, int, cudaStream_t);
 template void k5_launch_m<4>(const DevConsts&, int, const MulScratch&, uint64_t*, int, cudaStream_t);

@@ -22,20 +22,13 @@ void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int 
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st) {
     // K1: INTT over Q of [a1, b1, a2, b2], stored as y_i = [x_i (Q/q_i)^-1]_{q_i}
     ntt_inv(dc, PairQRowsP{pb, dc.logn, dc.nq}, QHatRowsIO{m.sa, dc.logn, dc.nq, dc.q2r_fold}, count * 4 * dc.nq, st);
-    if (count <= dc.shape.fuse_q2r_pairs) {
-        // K3's loader extends them to R
-#define L_Q2R(M) q2r_ntt_launch_m<M>(dc, m.sa, m.sb, count * 4, st)
-        DISPATCH_MAXQ(dc.nq, L_Q2R);
-#undef L_Q2R
-    } else {
-        // K2: Q -> R (centred)
+    // K2: Q -> R (centred)
 #define L_K2(K) k2_launch_m<K>(dc, m.sa, m.sb, count * 4, st)
-        DISPATCH_KS(dc.mm_ks, L_K2);
+    DISPATCH_KS(dc.mm_ks, L_K2);
 #undef L_K2
-        // K3: NTT over R in place, fully reduced (the tensor's products use barrett_prod)
-        ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sb, dc.idx_r, dc.nr), rows_io(dc, m.sb, dc.idx_r, dc.nr),
-                                       count * 4 * dc.nr, st);
-    }
+    // K3: NTT over R in place, fully reduced (the tensor's products use barrett_prod)
+    ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sb, dc.idx_r, dc.nr), rows_io(dc, m.sb, dc.idx_r, dc.nr),
+                                   count * 4 * dc.nr, st);
     // K4: tensor (Q part from the NTT-form inputs, R part from K3) fused into INTT over Q|R
     TensorSrc ts{pb, m.sb, dc};
     ntt_inv(dc, ts, QRFoldRowsIO{m.sc, dc.logn, dc.nq, dc.nqr, dc.idx_r, dc.qr_fold}, count * 3 * dc.nqr, st);

@@ -450,10 +450,6 @@ template <int KS>
 void bconv_mma_launch_m(const DevConsts& dc, bool q2r, const uint64_t* in, uint64_t* out, int polys, cudaStream_t st);
 template <int KS>
 void k5_launch_m(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st);
-// K3 with the Q -> R base extension in its loader: `polys` polynomials of y
-// rows over Q (QHatRowsIO layout) -> NTT-form R limbs, fully reduced
-template <int MAXQ>
-void q2r_ntt_launch_m(const DevConsts& dc, const uint64_t* y, uint64_t* out, int polys, cudaStream_t st);
 // K5: scale-and-round, R -> Q and (mode 1) the key-switch digit lift
 void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st);
 // the key-switch lift of the digits' own limbs in sd2 ([item][dnum][npq]) into every other prime of Q|P (lift.cu)

@@ -13,9 +13,8 @@ Knobs (include/kbfv.h, ``kbfv_tune_knob``):
   (CTA size of the Q -> R base conversion), ``k5_threads`` (CTA size of the
   scale-and-round / R -> Q / digit-lift kernels) and ``k5_fused_pairs``
   (batches of at most this many pairs run those as one kernel), ``bconv_cpt``
-  (coefficients per thread of the base conversion) and ``fuse_q2r_pairs``
-  (batches of at most this many pairs run the Q -> R base extension in the
-  loader of the forward NTT over R, no separate base-conversion launch),
+  (coefficients per thread of the standalone base conversions),
+  ``fuse_q2r_pairs`` (accepted without effect, see include/kbfv.h),
   ``l2_prefetch`` (NTT block kernels ask L2 for the block one wave ahead)
   ``split_rows_alone`` (``split_rows`` for multiplies that run as one
   stream, where no sibling sub-batch fills idle SMs) and ``min_branch_pairs``
