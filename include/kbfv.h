@@ -270,8 +270,9 @@ typedef enum {
     KBFV_TUNE_HOST_CHUNK = 2,    /* 0..128 (default 0 = ~32 MiB of inputs): pairs per chunk of
                                     kbfv_mul_relin_host when its chunk_pairs is 0 */
     KBFV_TUNE_SPLIT_ROWS = 3,    /* 0..2^20 (default 48): at N = 2^14, transforms of at most this
-                                    many rows (inside the multiply pipeline too) run as a radix-4
-                                    column pass and 2^12-point blocks instead of one block per row */
+                                    many rows (inside the multiply pipeline too) that are too many
+                                    for a cluster of CTAs per row run as a radix-4 column pass and
+                                    2^12-point blocks instead of one block per row */
     KBFV_TUNE_BCONV_THREADS = 4, /* 64, 128, 256 (default) or 512: CTA size of the base conversion
                                     Q -> R (the multiply's K2 and kbfv_bconv_*) */
     KBFV_TUNE_K5_THREADS = 5,    /* 64, 128 (default) or 256: CTA size of the multiply's

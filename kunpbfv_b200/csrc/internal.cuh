@@ -22,6 +22,7 @@
 #include "host_math.hpp"
 #include "kernels.cuh"
 #include "ntt.cuh"
+#include "ntt_cluster.cuh"
 #include "klss.cuh"
 
 using namespace kbfv;
@@ -110,6 +111,63 @@ static inline int resident_ctas_at(const void* kernel, int threads, int smem, in
     return cache[i];
 }
 
+// A launch of clusters of `cluster` CTAs. `early`: it may start while the kernel
+// before it on the stream still runs (programmatic dependent launch; the kernel
+// waits before it touches memory that other kernels use).
+template <class... P, class... A>
+static void launch_clusters(bool early, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                            unsigned cluster, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 2 : 1;
+    KB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
+// Whether a launch of `rows` rows runs on clusters (ntt_cluster.cuh): where that
+// takes less time than the other forms (148 SMs; us, cluster / other):
+//   2^12: 128 rows 9.3 / 10.4, 148 rows 13.1 / 10.4      2^13: 128 rows 15.2 / 16.6, 148 rows 17.8 / 16.6
+//   2^14: 8 rows 9.5 / 14.4, 26 rows 17 / 14.4 (the split form's single wave of up to
+//         148 quarter-row CTAs, against more than one cluster CTA per SM),
+//         40 rows 17 / 21.6, 64 rows 17 / 29, 112 rows 28 / 29, 128 rows 31 / 29
+//   2^15: 8 rows 11 / 18, 16 rows 17-22 / 17             2^16: never (4 rows 19 / 17)
+// Beside a sibling sub-batch the SMs that few rows leave idle are partly used and
+// the limits lie lower, at 2^14 most of all (8 pairs, 7 digits: 447 us with a
+// limit of 32, 469 with 96); a launch that waits early there holds SMs that the
+// sibling could use, so only launches alone on the GPU start early.
+static inline bool cluster_rows(const DevConsts& dc, int rows) {
+    const bool alone = dc.shape.tail_sms > 0;
+    switch (dc.logn) {
+        case 12:
+        case 13: return rows <= (alone ? 128 : 96);
+        case 14: return alone ? rows <= 18 || (rows > 37 && rows <= 112) : rows <= 32;
+        case 15: return rows <= 8;
+        default: return false;
+    }
+}
+template <int LOGN, class Src, class Dst, bool FULL>
+static void launch_fwd_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
+    using SH = ClusterShape<LOGN>;
+    static_assert(SH::SMEM_BYTES <= 48 << 10, "no attribute needed");
+    launch_clusters(dc.shape.tail_sms > 0, ntt_fwd_cluster_kernel<LOGN, Src, Dst, FULL>, (unsigned)rows << kClusterLog,
+                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_fwd, dc.mods);
+}
+template <int LOGN, class Src, class Dst>
+static void launch_inv_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
+    using SH = ClusterShape<LOGN>;
+    launch_clusters(dc.shape.tail_sms > 0, ntt_inv_cluster_kernel<LOGN, Src, Dst>, (unsigned)rows << kClusterLog,
+                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_inv, dc.mods);
+}
+
 template <int LOGB, class Src, class Dst, bool FULL = true>
 static void launch_fwd_block(const DevConsts& dc, Src s, Dst d, int rows, int logn, cudaStream_t st) {
     constexpr int SMEM = BlockShape<LOGB>::SMEM_BYTES;
@@ -179,8 +237,8 @@ static inline bool split14(const LaunchShape& sh, int rows) {
     return waves >= 2 && waves <= 5 && rows - (waves - 1) * sh.tail_sms <= 96 - 14 * (waves - 1);
 }
 
-// Forward NTT of `rows` rows read through `s` and written through `d`.
-// For logn <= 14 one block kernel (N = 2^14 with at most shape.split_rows14 rows:
+// Forward NTT of `rows` rows read through `s` and written through `d`. Few rows of
+// 2^12..2^15 points run on clusters (cluster_rows). Else, for logn <= 14 one block kernel (N = 2^14 with at most shape.split_rows14 rows:
 // as for 15/16 with a radix-4 column pass); for 15/16 a radix-8/16 column pass
 // (s -> plain_of(d)) then 2^12-point block kernels from plain_of(d) to d in
 // place (d must also be readable): several 256-thread CTAs per SM run faster
@@ -189,6 +247,16 @@ static inline bool split14(const LaunchShape& sh, int rows) {
 template <class Src, class Dst, bool FULL = true>
 static void ntt_fwd(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
     if (rows <= 0) return;
+    if (cluster_rows(dc, rows)) {
+        switch (dc.logn) {
+            case 12: launch_fwd_cluster<12, Src, Dst, FULL>(dc, s, d, rows, st); break;
+            case 13: launch_fwd_cluster<13, Src, Dst, FULL>(dc, s, d, rows, st); break;
+            case 14: launch_fwd_cluster<14, Src, Dst, FULL>(dc, s, d, rows, st); break;
+            default: launch_fwd_cluster<15, Src, Dst, FULL>(dc, s, d, rows, st); break;
+        }
+        check_launch("ntt_fwd");
+        return;
+    }
     switch (dc.logn) {
         case 10: launch_fwd_block<10, Src, Dst, FULL>(dc, s, d, rows, 10, st); break;
         case 11: launch_fwd_block<11, Src, Dst, FULL>(dc, s, d, rows, 11, st); break;
@@ -230,6 +298,16 @@ static void ntt_fwd(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st
 template <class Src, class Dst>
 static void ntt_inv(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
     if (rows <= 0) return;
+    if (cluster_rows(dc, rows)) {
+        switch (dc.logn) {
+            case 12: launch_inv_cluster<12>(dc, s, d, rows, st); break;
+            case 13: launch_inv_cluster<13>(dc, s, d, rows, st); break;
+            case 14: launch_inv_cluster<14>(dc, s, d, rows, st); break;
+            default: launch_inv_cluster<15>(dc, s, d, rows, st); break;
+        }
+        check_launch("ntt_inv");
+        return;
+    }
     switch (dc.logn) {
         case 10: launch_inv_block<10, Src, Dst, true>(dc, s, d, rows, 10, st); break;
         case 11: launch_inv_block<11, Src, Dst, true>(dc, s, d, rows, 11, st); break;

@@ -124,8 +124,8 @@ struct ExtProdRow {
             uint64_t a[K], b[K];
 #pragma unroll
             for (int i = 0; i < K; i++) {
-                a[i] = __ldg(dig + d * ds + j[i]);
-                b[i] = __ldg(key + d * ks + j[i]);
+                a[i] = dig[d * ds + j[i]];
+                b[i] = key[d * ks + j[i]];
             }
 #pragma unroll
             for (int i = 0; i < K; i++) mac(acc[i], a[i], b[i]);

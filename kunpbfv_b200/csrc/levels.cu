@@ -52,7 +52,7 @@ struct ModSwitchOutRow {
     __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
         uint64_t x[K];
 #pragma unroll
-        for (int i = 0; i < K; i++) x[i] = __ldg(ct + j[i]);
+        for (int i = 0; i < K; i++) x[i] = ct[j[i]];
 #pragma unroll
         for (int i = 0; i < K; i++) out[j[i]] = shoup(x[i] + (q << 3) - v[i], w, ws, q);
     }

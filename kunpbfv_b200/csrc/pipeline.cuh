@@ -45,17 +45,16 @@ struct QRFoldRowsIO {
 };
 
 // K4 source: tensor product of the pair at limb l of Q|R, one of three outputs
-// values in [0, 4q), as the inverse transform takes them; the loads are read-only ones: no store
-// of the kernel holds them back
+// values in [0, 4q), as the inverse transform takes them
 struct TensorRow {
     const uint64_t *a1, *b1, *a2, *b2;
     int k;
     uint64_t q, mh;  // mh: barrett_prod constant (inputs are fully reduced)
     __device__ __forceinline__ uint64_t load(int j) const {
-        if (k == 0) return barrett_prod_lazy(mul_wide(__ldg(a1 + j), __ldg(a2 + j)), q, mh);
-        if (k == 2) return barrett_prod_lazy(mul_wide(__ldg(b1 + j), __ldg(b2 + j)), q, mh);
-        u128 acc = mul_wide(__ldg(a1 + j), __ldg(b2 + j));
-        mac(acc, __ldg(b1 + j), __ldg(a2 + j));  // < 2 q^2
+        if (k == 0) return barrett_prod_lazy(mul_wide(a1[j], a2[j]), q, mh);
+        if (k == 2) return barrett_prod_lazy(mul_wide(b1[j], b2[j]), q, mh);
+        u128 acc = mul_wide(a1[j], b2[j]);
+        mac(acc, b1[j], a2[j]);  // < 2 q^2
         return barrett_prod_lazy(acc, q, mh);
     }
     __device__ __forceinline__ void store(int, uint64_t) const {}
@@ -92,7 +91,8 @@ struct TensorSrc {
 
 // sum_d digit_d * key_d at K points: [0, 4q) for one digit (fully reduced
 // factors), else [0, q). All points' operands of a digit are loaded before they
-// are used, by read-only loads.
+// are used. (Ordinary loads: a kernel that starts before its predecessor ends must
+// not read the predecessor's results through the read-only path.)
 template <int K>
 __device__ __forceinline__ void key_product(const uint64_t* dig, const uint64_t* key, size_t ds, size_t ks, int ndig,
                                             uint64_t q, uint64_t mh, uint64_t ml, uint64_t mp, const int (&j)[K],
@@ -101,8 +101,8 @@ __device__ __forceinline__ void key_product(const uint64_t* dig, const uint64_t*
     if (ndig == 1) {
 #pragma unroll
         for (int i = 0; i < K; i++) {
-            a[i] = __ldg(dig + j[i]);
-            b[i] = __ldg(key + j[i]);
+            a[i] = dig[j[i]];
+            b[i] = key[j[i]];
         }
 #pragma unroll
         for (int i = 0; i < K; i++) x[i] = barrett_prod_lazy(mul_wide(a[i], b[i]), q, mp);
@@ -114,8 +114,8 @@ __device__ __forceinline__ void key_product(const uint64_t* dig, const uint64_t*
     for (int d = 0; d < ndig; d++, dig += ds, key += ks) {
 #pragma unroll
         for (int i = 0; i < K; i++) {
-            a[i] = __ldg(dig + j[i]);
-            b[i] = __ldg(key + j[i]);
+            a[i] = dig[j[i]];
+            b[i] = key[j[i]];
         }
 #pragma unroll
         for (int i = 0; i < K; i++) mac(acc[i], a[i], b[i]);
@@ -263,15 +263,15 @@ struct ModDownKeyRow {
         uint64_t y[K];
 #pragma unroll
         for (int i = 0; i < K; i++) {
-            y[i] = __ldg(xp + j[i]);
-            x[i] = add ? __ldg(add + j[i]) : 0;
+            y[i] = xp[j[i]];
+            x[i] = add ? add[j[i]] : 0;
         }
         for (int k = 0; k < np; k++) {
             if (k) {
 #pragma unroll
-                for (int i = 0; i < K; i++) y[i] = __ldg(xp + k * limb + j[i]);
+                for (int i = 0; i < K; i++) y[i] = xp[k * limb + j[i]];
             }
-            const ulonglong2 w = __ldg(c + k);
+            const ulonglong2 w = c[k];
 #pragma unroll
             for (int i = 0; i < K; i++) x[i] = csub63(x[i], q << 2) + shoup4(y[i], w.x, w.y, q);
         }
@@ -343,7 +343,7 @@ struct OutKeyRow {
         if (extra) {
             uint64_t e[K];
 #pragma unroll
-            for (int i = 0; i < K; i++) e[i] = __ldg(extra + j[i]);
+            for (int i = 0; i < K; i++) e[i] = extra[j[i]];
 #pragma unroll
             for (int i = 0; i < K; i++) ip[i] = add_mod(ip[i], e[i], q);
         }
@@ -407,7 +407,7 @@ struct DecSrc {
         uint64_t q, mh, ml;
         // a and s fully reduced: one-high-product Barrett (mh holds its constant); below 3q
         __device__ __forceinline__ uint64_t load(int j) const {
-            return csub63(barrett_prod_lazy(mul_wide(__ldg(a + j), __ldg(s + j)), q, mh), q << 1) + __ldg(b + j);
+            return csub63(barrett_prod_lazy(mul_wide(a[j], s[j]), q, mh), q << 1) + b[j];
         }
         __device__ __forceinline__ void store(int, uint64_t) const {}
     };

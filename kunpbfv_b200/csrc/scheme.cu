@@ -166,8 +166,8 @@ struct EncOutRow {
         uint64_t a[K], b[K];
 #pragma unroll
         for (int i = 0; i < K; i++) {
-            a[i] = __ldg(v + j[i]);
-            b[i] = __ldg(pk + j[i]);
+            a[i] = v[j[i]];
+            b[i] = pk[j[i]];
         }
 #pragma unroll
         for (int i = 0; i < K; i++)
@@ -264,7 +264,7 @@ struct DecSrcP {
         const uint64_t *a, *b, *s;
         uint64_t q, mp;
         __device__ __forceinline__ uint64_t load(int j) const {  // below 3q, as DecSrc
-            return csub63(barrett_prod_lazy(mul_wide(__ldg(a + j), __ldg(s + j)), q, mp), q << 1) + __ldg(b + j);
+            return csub63(barrett_prod_lazy(mul_wide(a[j], s[j]), q, mp), q << 1) + b[j];
         }
         __device__ __forceinline__ void store(int, uint64_t) const {}
     };
