@@ -577,7 +577,7 @@ uint8_t* ensure_scratch(Context& c, size_t bytes) {
 // 5: 128-bit Barrett, 6: one-high-product Barrett, 7: 32x32->64 multiply-add,
 // 8: 32x32 high product, 9: 32-bit multiply-add, 10: mac32 (64x64->128
 // multiply-accumulate from 32-bit partial products), 11: forward butterfly
-// with shoup4_32 (the NTT kernels' butterfly), 12: 32-bit multiply-add issue
+// with shoup4_wide (the NTT kernels' butterfly), 12: 32-bit multiply-add issue
 // rate (16 dependent mad.lo.u32 per chain step, the IMAD pipe's peak),
 // 13: 32x32->64 multiply-add issue rate (16 dependent mad.wide.u32 per step),
 // 14: 60x60-bit multiply-accumulate from 30-bit halves (mac30: four
@@ -653,7 +653,7 @@ __global__ void probe_arith_kernel(uint64_t* out, int iters, uint64_t q, uint64_
                 for (int u = 0; u < kImadPerStep; u++) asm("mad.hi.u32 %0, %0, %1, %2;" : "+r"(x) : "r"(m), "r"(k));
                 acc[c].lo = x;
             }
-            if (KIND == 11) {  // the NTT kernels' butterfly (Shoup product from 32-bit multiplies)
+            if (KIND == 11) {  // the NTT kernels' butterfly (shoup4_wide)
                 uint64_t x = a[c], y = b[c];
                 ct_bfly(x, y, tw_t{b[c], a[c]}, q, q << 2);
                 acc[c].lo += x ^ y;
