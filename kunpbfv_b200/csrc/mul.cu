@@ -3,6 +3,7 @@
 // allocation-free variant.
 #include <cuda.h>
 
+#include "key_ip.cuh"
 #include "pipeline.cuh"
 
 // Key-switch tail over NTT-form digits (sd2, [item][ndig][npq]) and a key
@@ -11,9 +12,34 @@
 // Only the P limbs of x are brought back to coefficient form (inverse NTT over
 // P, the key product fused into its loads) for the conversion to Q. The Q limbs
 // stay in the NTT domain, where the forward NTT's store adds them:
-//   NTT(add - P^-1 [x_P]_Q) + P^-1 x_Q,  with x_Q computed at the store.
+//   NTT(add - P^-1 [x_P]_Q) + P^-1 x_Q,  with x_Q computed (or, from four digits
+// on, read) at the store.
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
                     const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st, const KsExtra& ex) {
+    if (ndig >= 4) {
+        // From four digits on the products are summed apart (key_ip.cuh), times P^-1
+        // on the Q limbs: a point's digits are read once for both outputs and the
+        // sums written and read again (ndig + 4 accesses of the batch's own data
+        // against 2 ndig inside the transforms, and the key once for up to four
+        // items). us, summed apart / inside: N = 16384, 7 digits, 1 item 52 / 66,
+        // 8 items 217 / 263, 64 items 1368 / 1367; 2 digits, 64 items 1001 / 956;
+        // N = 32768, 3 digits, 4 items 284 / 295, 64 items 3571 / 3433.
+        const size_t n = (size_t)1 << dc.logn;
+        KeyIpJob J{};
+        J.dig = sd2; J.key = key; J.out = se;
+        J.dig_d = (size_t)dc.npq * n; J.dig_item = ndig * J.dig_d;
+        J.key_o = (size_t)dc.key_npq * n; J.key_d = 2 * J.key_o;
+        J.out_o = (size_t)dc.npq * n; J.out_item = 2 * J.out_o;
+        J.ndig = ndig; J.items = count; J.outputs = 2; J.limbs = dc.npq;
+        J.nq = dc.nq; J.key_gap = dc.key_nq - dc.nq;
+        J.scale = dc.pinv_q; J.scales = dc.pinv_qs;
+        J.extra = ex.base; J.extra_item = ex.stride; J.extra_o = (size_t)dc.nq * n; J.extra_from = ex.from;
+        key_ip_launch<2>(dc, J, st);
+        const SeFoldRowsP sp{se, dc.logn, dc.nq, dc.np, dc.npq, dc.p_fold};
+        ntt_inv(dc, sp, sp, count * 2 * dc.np, st);
+        ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtSumDst{pb, se, dc}, count * 2 * dc.nq, st);
+        return;
+    }
     ntt_inv(dc, KeyIPSrc{sd2, key, dc, ndig, dc.nq, dc.np}, SeFoldRowsP{se, dc.logn, dc.nq, dc.np, dc.npq, dc.p_fold},
             count * 2 * dc.np, st);
     ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtKeyDst{pb, sd2, key, dc, ndig, ex}, count * 2 * dc.nq, st);

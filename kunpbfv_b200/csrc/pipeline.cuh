@@ -382,6 +382,35 @@ struct OutCtKeyDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
         return r;
     }
 };
+// The same over a key product that key_ip.cuh has summed and scaled by P^-1
+// (limb l of se's Q part)
+struct OutSumRow {
+    static constexpr bool kStoreMany = true;
+    uint64_t* p;
+    const uint64_t* x;
+    uint64_t q;
+    // v below 8q
+    template <int K>
+    __device__ __forceinline__ void store_n(const int (&j)[K], const uint64_t (&v)[K]) const {
+        uint64_t y[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) y[i] = x[j[i]];
+#pragma unroll
+        for (int i = 0; i < K; i++) p[j[i]] = reduce_from(csub63(v[i], q << 2) + y[i], q, 3);
+    }
+};
+struct OutCtSumDst {  // rows: (item, h, l) -> out[item] + (h*nq + l)*N
+    PtrBatch pb;
+    const uint64_t* se;  // [item][2][npq]
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.nq; }
+    __device__ __forceinline__ OutSumRow bind(int row) const {
+        const int nq = dc.nq, logn = dc.logn;
+        const int item = row / (2 * nq), w = row % (2 * nq), h = w / nq, l = w % nq;
+        return OutSumRow{pb.o[item] + ((size_t)w << logn), se + (((size_t)(item * 2 + h) * dc.npq + l) << logn), dc.mods[l]};
+    }
+};
+static inline OutCtDst plain_of(const OutCtSumDst& d) { return OutCtDst{d.pb, d.dc.logn, d.dc.nq}; }
 // the column pass of a split transform writes plain values; only the block
 // kernel's final store runs the epilogue
 static inline OutCtDst plain_of(const OutCtKeyDst& d) { return OutCtDst{d.pb, d.dc.logn, d.dc.nq}; }

@@ -1,0 +1,71 @@
+"""Key switches of four digits and more, whose products with the key are summed
+by a kernel of their own: every number of items that a thread takes (1..4, and
+groups with a short last one), the smallest ring and split ones, the added term on
+both halves (relinearisation) and on one (rotation), and a level's live primes of
+the top level's key, against the oracle, bit for bit."""
+import numpy as np
+import pytest
+
+from tests.gpu_util import dev, host, make_pair, rand_rows
+
+pytestmark = pytest.mark.gpu
+
+SEED = bytes(range(5, 37))
+
+
+def _relinearize(ctx, rlk, tensors):
+    import torch
+    from kunpbfv_b200.api import _check, _ptr, _stream_ptr, lib
+    out = torch.full((len(tensors), 2, ctx.q_count, ctx.N), -1, dtype=torch.int64, device="cuda")
+    d, k = dev(tensors), dev(rlk)
+    _check(lib().kbfv_relinearize(ctx.handle, _ptr(k), _ptr(d), _ptr(out), len(tensors), _stream_ptr(None)))
+    return host(out).reshape(len(tensors), 2, ctx.q_count, ctx.N)
+
+
+@pytest.mark.parametrize("log_n,nq,np_,dnum,items", [(10, 4, 1, 4, 1), (12, 5, 1, 5, 2), (13, 8, 2, 4, 3), (14, 7, 1, 7, 4),
+                                                     (12, 7, 1, 7, 5), (15, 4, 1, 4, 9), (12, 3, 1, 3, 5)])
+def test_relinearize_digits(log_n, nq, np_, dnum, items):
+    import oracle
+    ps = oracle.primes_bits(1 << log_n, 60, nq + np_)
+    ctx, orc = make_pair(log_n, ps[np_:], ps[:np_], dnum)
+    n, npq = ctx.N, nq + np_
+    rlk = rand_rows(orc, list(range(npq)) * 2 * dnum, n, 1).reshape(dnum, 2, npq, n)
+    d = rand_rows(orc, list(range(nq)) * 3 * items, n, 2).reshape(items, 3, nq, n)
+    top = np.array(orc.primes[:npq], dtype=np.uint64) - 1
+    rlk[:, :, :, 0] = top          # the largest residues throughout
+    d[:, :, :, 0] = top[:nq]
+    got = _relinearize(ctx, rlk, d)
+    for i in sorted({0, items // 2, items - 1}):
+        assert np.array_equal(got[i], orc.relinearize(d[i], rlk)), i
+
+
+def test_rotation_and_level():
+    import kunpbfv_b200 as kb
+    import oracle
+    T = 65537
+    ps = oracle.primes_bits(1 << 12, 50, 10)
+    q, p = ps[2:], ps[:2]
+    ctx, top = make_pair(12, q, p, 4)
+    sk = kb.SecretKey(ctx, SEED)
+    sch = kb.BFVScheme(ctx, SEED)
+    sch.addEncKey(sk)
+    sch.addMultKey_23(sk)
+    sch.addLeftRotKey_23(sk, 1)
+    osk = top.keygen_secret(SEED)
+    g = sch.galois_element(1)
+    ogk = top.keygen_galois(SEED, osk, g)
+    orlk = top.keygen_relin(SEED, osk)
+    v = np.random.default_rng(4).integers(0, T, size=(5, ctx.N), dtype=np.uint64)
+    ct = sch.encryptMsg(kb.Plaintext(ctx, ctx.encode(dev(v))), enc_id=3)
+    h = host(ct.cipher_device).reshape(5, 2, 8, ctx.N)
+    got = host(sch.apply_galois(ct, g).cipher_device).reshape(h.shape)
+    for i in (0, 4):
+        assert np.array_equal(got[i], top.apply_galois(ogk, g, h[i])), i
+    c7 = sch.mod_switch(ct)  # 7 live primes: digits 2, 2, 2, 1
+    o7 = oracle.Oracle(12, T, q[:7], p, alpha=2)
+    rl = np.stack([np.stack([np.concatenate([orlk[d][k][:7], orlk[d][k][8:]]) for k in range(2)]) for d in range(o7.dnum)])
+    assert o7.dnum == 4
+    h7 = host(c7.cipher_device).reshape(5, 2, 7, ctx.N)
+    sq = host(sch.mult_relin(c7, c7).cipher_device).reshape(5, 2, 7, ctx.N)
+    for i in (0, 4):
+        assert np.array_equal(sq[i], o7.mul_relin(h7[i], h7[i], rl)), i
