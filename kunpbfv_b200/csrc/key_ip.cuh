@@ -18,7 +18,8 @@ struct KeyIpJob {
     const uint64_t* dig;  // item 0, digit 0, limb 0; limbs adjacent
     const uint64_t* key;  // output 0, digit 0, limb 0
     uint64_t* out;
-    size_t dig_item, dig_d, key_o, key_d, out_item, out_o;  // strides in words
+    size_t dig_item, dig_d, key_o, key_half, key_d, out_item, out_o;  // strides in words
+    int per_half;         // output o is number o % per_half of key half o / per_half
     int ndig, items, outputs, limbs;
     int prime0;           // limb m uses prime prime0 + m
     int nq, key_gap;      // limbs from nq on lie key_gap limbs further in the key (a level's key is the top's)
@@ -41,7 +42,10 @@ static __global__ void __launch_bounds__(256, C * O > 8 ? 2 : 3) key_ip_kernel(K
 #pragma unroll
     for (int i = 0; i < C; i++) dig[i] = J.dig + (size_t)min(i0 + i, J.items - 1) * J.dig_item + at;
 #pragma unroll
-    for (int o = 0; o < O; o++) key[o] = J.key + (size_t)min(o0 + o, J.outputs - 1) * J.key_o + kat;
+    for (int o = 0; o < O; o++) {
+        const int w = min(o0 + o, J.outputs - 1);
+        key[o] = J.key + (size_t)(w / J.per_half) * J.key_half + (size_t)(w % J.per_half) * J.key_o + kat;
+    }
     u128 acc[C][O];
 #pragma unroll
     for (int i = 0; i < C; i++)

@@ -1,6 +1,53 @@
 // libkbfv: the reference's key switch over the auxiliary T base (KLSS) and its
 // pieces as entry points.
+#include "key_ip.cuh"
 #include "pipeline.cuh"
+
+// blocks of at most 1, 2, 4, 8 or 16 primes; 4, 8 or 12 T primes
+static void klss_block_to_t(const DevConsts& dc, const KlssConsts& kc, const uint64_t* in, uint64_t* out, int which,
+                            size_t in_stride, size_t out_stride, unsigned items, cudaStream_t st) {
+    const dim3 grid((1u << dc.logn) / 256, (unsigned)(which == 0 ? kc.nqj : kc.nri), items);
+    const int w = which == 0 ? dc.np : kc.gamma;
+#define L_BT(W) klss_block_to_t_kernel<W><<<grid, 128, 0, st>>>(dc, kc, in, out, which, in_stride, out_stride)
+    if (w <= 1) L_BT(1);
+    else if (w <= 2) L_BT(2);
+    else if (w <= 4) L_BT(4);
+    else if (w <= 8) L_BT(8);
+    else L_BT(kMaxBlk);
+#undef L_BT
+    check_launch("klss_block_to_t");
+}
+static void klss_t_to_pq(const DevConsts& dc, const KlssConsts& kc, const uint64_t* in, uint64_t* out, unsigned polys,
+                         cudaStream_t st) {
+    const dim3 grid((1u << dc.logn) / 256, (unsigned)kc.nri, polys);
+#define L_TP(N) klss_t_to_pq_kernel<N><<<grid, 128, 0, st>>>(dc, kc, in, out)
+    if (kc.nt <= 4) L_TP(4);
+    else if (kc.nt <= 8) L_TP(8);
+    else L_TP(kMaxT);
+#undef L_TP
+    check_launch("klss_t_to_pq");
+}
+
+// External product over T of `count` items, NTT form: out[item][h][block][t] =
+// sum over digits i of dig[item][i][t] * key[h][i][block][t] mod t_t.
+// Inside the inverse transform's loads, 8 rows of every T prime read each digit again
+// and 6 each key limb, 755 MB of L2 reads for 3 items of 15 digits and 4 blocks at N
+// = 32768: 147 us with the transform's block pass. Summed apart (key_ip.cuh) 63 + 37
+// us, 27 of the 63 for the multiply-accumulates and 19 for the key from HBM. Four
+// outputs a thread: with two, every digit is read four times (13 us more).
+static void klss_ext_product(const DevConsts& dc, const KlssConsts& kc, const uint64_t* dig, const uint64_t* key,
+                             uint64_t* out, int count, cudaStream_t st) {
+    const size_t n = (size_t)1 << dc.logn, row = (size_t)kc.nt * n;
+    KeyIpJob J{};
+    J.dig = dig; J.key = key; J.out = out;
+    J.dig_d = row; J.dig_item = kc.nqj * row;
+    J.key_d = kc.nri * row;
+    J.key_o = row; J.key_half = kc.nqj * J.key_d; J.per_half = kc.nri;
+    J.out_o = row; J.out_item = (size_t)2 * kc.nri * row;
+    J.ndig = kc.nqj; J.items = count; J.outputs = 2 * kc.nri; J.limbs = kc.nt;
+    J.prime0 = dc.idx_t; J.nq = kc.nt;
+    key_ip_launch<4>(dc, J, st);
+}
 
 // T-base key switch (the reference's KLSS, include/KeySwitch_23.cuh:244-330) of
 // a1*a2 given in coefficient form over Q (sd2, [item][nq]); writes the P|Q
@@ -9,19 +56,15 @@ static void klss_keyswitch(Context& c, const uint64_t* rlk_t, int count, const M
     const DevConsts& dc = c.dc;
     const KlssConsts& kc = c.kc;
     // Qj blocks -> T (modUpQjtoT_23)
-    klss_block_to_t_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)kc.nqj, (unsigned)count), 128, 0, st>>>(
-        dc, kc, m.sd2, m.st1, 0, (size_t)c.nq << c.logn, (size_t)kc.nqj * c.nt << c.logn);
-    check_launch("klss_qj_to_t");
+    klss_block_to_t(dc, kc, m.sd2, m.st1, 0, (size_t)c.nq << c.logn, (size_t)kc.nqj * c.nt << c.logn, (unsigned)count, st);
     // NTT over T
     ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.st1, dc.idx_t, c.nt), rows_io(dc, m.st1, dc.idx_t, c.nt),
                                    count * kc.nqj * c.nt, st);
-    // external product over T fused into INTT over T (external_product_T)
-    ntt_inv(dc, ExtProdSrc{m.st1, rlk_t, dc, c.nt, kc.nri, kc.nqj, kc.nqj}, rows_io(dc, m.st2, dc.idx_t, c.nt),
-            count * 2 * kc.nri * c.nt, st);
+    // external product over T (external_product_T) and INTT over T
+    klss_ext_product(dc, kc, m.st1, rlk_t, m.st2, count, st);
+    ntt_inv(dc, rows_io(dc, m.st2, dc.idx_t, c.nt), rows_io(dc, m.st2, dc.idx_t, c.nt), count * 2 * kc.nri * c.nt, st);
     // centred T -> P|Q (modUpTtoPQl_23)
-    klss_t_to_pq_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)kc.nri, (unsigned)(count * 2)), 128, 0, st>>>(
-        dc, kc, m.st2, m.se);
-    check_launch("klss_t_to_pq");
+    klss_t_to_pq(dc, kc, m.st2, m.se, (unsigned)(count * 2), st);
 }
 
 static void mul_relin_klss_chunk(Context& c, const uint64_t* rlk_t, const PtrBatch& pb, int count,
@@ -62,10 +105,9 @@ int kbfv_rlk_to_klss(kbfv_context* ctx, const uint64_t* d_rlk, uint64_t* d_rlk_t
                 c.dnum * 2 * npq, st);
         // Ri blocks -> T (modUpPQtoT_23), written as [a|b][digit][Ri][T]
         for (int h = 0; h < 2; h++) {
-            klss_block_to_t_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)kc.nri, (unsigned)c.dnum), 128, 0, st>>>(
-                dc, kc, coef + ((size_t)h * npq << c.logn), d_rlk_t + ((size_t)h * c.dnum * kc.nri * c.nt << c.logn), 1,
-                (size_t)2 * npq << c.logn, (size_t)kc.nri * c.nt << c.logn);
-            check_launch("klss_pq_to_t");
+            klss_block_to_t(dc, kc, coef + ((size_t)h * npq << c.logn),
+                            d_rlk_t + ((size_t)h * c.dnum * kc.nri * c.nt << c.logn), 1, (size_t)2 * npq << c.logn,
+                            (size_t)kc.nri * c.nt << c.logn, (unsigned)c.dnum, st);
         }
         RowsIO io = rows_io(dc, d_rlk_t, dc.idx_t, c.nt);
         ntt_fwd(dc, io, io, 2 * c.dnum * kc.nri * c.nt, st);
@@ -80,9 +122,8 @@ int kbfv_klss_modup_qj_to_t(kbfv_context* ctx, const uint64_t* d_in, uint64_t* d
         require_klss(c);
         KB_REQUIRE(polys <= 65535, KBFV_ERR_INVALID, "at most 65535 polynomials per call");
         if (!polys) return;
-        klss_block_to_t_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)c.kc.nqj, polys), 128, 0, S(stream)>>>(
-            c.dc, c.kc, d_in, d_out, 0, (size_t)c.nq << c.logn, (size_t)c.kc.nqj * c.nt << c.logn);
-        check_launch("klss_qj_to_t");
+        klss_block_to_t(c.dc, c.kc, d_in, d_out, 0, (size_t)c.nq << c.logn, (size_t)c.kc.nqj * c.nt << c.logn, polys,
+                        S(stream));
     });
 }
 
@@ -94,9 +135,8 @@ int kbfv_klss_modup_pq_to_t(kbfv_context* ctx, const uint64_t* d_in, uint64_t* d
         require_klss(c);
         KB_REQUIRE(polys <= 65535, KBFV_ERR_INVALID, "at most 65535 polynomials per call");
         if (!polys) return;
-        klss_block_to_t_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)c.kc.nri, polys), 128, 0, S(stream)>>>(
-            c.dc, c.kc, d_in, d_out, 1, (size_t)c.dc.npq << c.logn, (size_t)c.kc.nri * c.nt << c.logn);
-        check_launch("klss_pq_to_t");
+        klss_block_to_t(c.dc, c.kc, d_in, d_out, 1, (size_t)c.dc.npq << c.logn, (size_t)c.kc.nri * c.nt << c.logn, polys,
+                        S(stream));
     });
 }
 
@@ -108,8 +148,9 @@ int kbfv_klss_external_product(kbfv_context* ctx, const uint64_t* d_digits, cons
         require_klss(c);
         KB_REQUIRE(d_rlk_t, KBFV_ERR_NO_KEY, "T-base relinearisation key missing");
         const KlssConsts& kc = c.kc;
-        ntt_inv(c.dc, ExtProdSrc{d_digits, d_rlk_t, c.dc, c.nt, kc.nri, kc.nqj, kc.nqj},
-                rows_io(c.dc, d_out, c.dc.idx_t, c.nt), (int)count * 2 * kc.nri * c.nt, S(stream));
+        klss_ext_product(c.dc, kc, d_digits, d_rlk_t, d_out, (int)count, S(stream));
+        ntt_inv(c.dc, rows_io(c.dc, d_out, c.dc.idx_t, c.nt), rows_io(c.dc, d_out, c.dc.idx_t, c.nt),
+                (int)count * 2 * kc.nri * c.nt, S(stream));
     });
 }
 
@@ -120,9 +161,7 @@ int kbfv_klss_t_to_pq(kbfv_context* ctx, const uint64_t* d_in, uint64_t* d_out, 
         require_klss(c);
         KB_REQUIRE(polys <= 65535, KBFV_ERR_INVALID, "at most 65535 polynomials per call");
         if (!polys) return;
-        klss_t_to_pq_kernel<<<dim3((unsigned)(c.n / 128), (unsigned)c.kc.nri, polys), 128, 0, S(stream)>>>(
-            c.dc, c.kc, d_in, d_out);
-        check_launch("klss_t_to_pq");
+        klss_t_to_pq(c.dc, c.kc, d_in, d_out, polys, S(stream));
     });
 }
 

@@ -28,7 +28,7 @@ void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int 
         KeyIpJob J{};
         J.dig = sd2; J.key = key; J.out = se;
         J.dig_d = (size_t)dc.npq * n; J.dig_item = ndig * J.dig_d;
-        J.key_o = (size_t)dc.key_npq * n; J.key_d = 2 * J.key_o;
+        J.key_half = (size_t)dc.key_npq * n; J.key_d = 2 * J.key_half; J.per_half = 1;
         J.out_o = (size_t)dc.npq * n; J.out_item = 2 * J.out_o;
         J.ndig = ndig; J.items = count; J.outputs = 2; J.limbs = dc.npq;
         J.nq = dc.nq; J.key_gap = dc.key_nq - dc.nq;
