@@ -92,6 +92,34 @@ struct has_store_n : std::false_type {};
 template <class T>
 struct has_store_n<T, std::enable_if_t<T::kStoreMany>> : std::true_type {};
 
+// A row that the inverse transform's first pass reads directly can take K adjacent
+// points at once (`load_adj<K>(j, x)`, j a multiple of K).
+template <class T, class = void>
+struct has_load_adj : std::false_type {};
+template <class T>
+struct has_load_adj<T, std::enable_if_t<T::kLoadAdj>> : std::true_type {};
+
+// K adjacent words, in 16-byte loads where the address allows: with 8-byte loads of
+// 32-byte lane strides every one of a lane's four loads goes through the L1's data
+// stage for the same lines again (## of the shared-memory and L1 cycles of the
+// kernel). The branch is the same for the whole CTA.
+__device__ __forceinline__ bool wide_ok(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+template <int K>
+__device__ __forceinline__ void load_adjacent(const uint64_t* p, bool wide, uint64_t* x) {
+    static_assert(K % 2 == 0, "pairs of words");
+    if (wide) {
+#pragma unroll
+        for (int k = 0; k < K; k += 2) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + k);
+            x[k] = v.x;
+            x[k + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) x[k] = p[k];
+    }
+}
+
 // x[k] = row value at index(k), k < K
 template <int K, class Row, class Index>
 __device__ __forceinline__ void load_points(const Row& s, uint64_t* x, Index index) {
@@ -451,7 +479,8 @@ __device__ __forceinline__ void inv_pass_load(const PassCtx& c, const SRow& s) {
     for (int g = 0; g < NG; g++) {
         const int lbase = adjacent_group<LOGB, R>(g, c.t) << R;
         uint64_t x[G];
-        load_points<G>(s, x, [&](int k) { return c.goff + lbase + k; });
+        if constexpr (has_load_adj<SRow>::value) s.template load_adj<G>(c.goff + lbase, x);
+        else load_points<G>(s, x, [&](int k) { return c.goff + lbase + k; });
         const int s0 = c.sbase + S0;
         inv_group<R>(x, c.tw, s0, (c.goff + lbase) >> (c.logn - s0), c.q, c.q4, false);
 #pragma unroll
@@ -671,7 +700,10 @@ ntt_inv_col16_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const ui
 // Row functors: prime(row), bind(row) -> {load(j), store(j, v)}
 // ---------------------------------------------------------------------------
 struct PtrRow {
+    static constexpr bool kLoadAdj = true;
     uint64_t* p;
+    template <int K>
+    __device__ __forceinline__ void load_adj(int j, uint64_t* x) const { load_adjacent<K>(p + j, wide_ok(p), x); }
     __device__ __forceinline__ void prefetch(int off, int n) const { l2_prefetch(p + off, (uint32_t)n * 8); }
     __device__ __forceinline__ uint64_t load(int j) const { return p[j]; }
     __device__ __forceinline__ void store(int j, uint64_t v) const { p[j] = v; }

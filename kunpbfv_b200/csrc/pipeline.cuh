@@ -47,8 +47,30 @@ struct QRFoldRowsIO {
 // K4 source: tensor product of the pair at limb l of Q|R, one of three outputs
 // values in [0, 4q), as the inverse transform takes them
 struct TensorRow {
+    static constexpr bool kLoadAdj = true;
     const uint64_t *a1, *b1, *a2, *b2;
     int k;
+    template <int K>
+    __device__ __forceinline__ void load_adj(int j, uint64_t* x) const {
+        const bool wide = wide_ok(a1) && wide_ok(b1) && wide_ok(a2) && wide_ok(b2);
+        uint64_t y[K];
+        load_adjacent<K>((k == 2 ? b1 : a1) + j, wide, x);
+        load_adjacent<K>((k == 0 ? a2 : b2) + j, wide, y);
+        if (k == 1) {
+            uint64_t u[K], v[K];
+            load_adjacent<K>(b1 + j, wide, u);
+            load_adjacent<K>(a2 + j, wide, v);
+#pragma unroll
+            for (int i = 0; i < K; i++) {
+                u128 acc = mul_wide(x[i], y[i]);
+                mac(acc, u[i], v[i]);  // < 2 q^2
+                x[i] = barrett_prod_lazy(acc, q, mh);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < K; i++) x[i] = barrett_prod_lazy(mul_wide(x[i], y[i]), q, mh);
+        }
+    }
     uint64_t q, mh;  // mh: barrett_prod constant (inputs are fully reduced)
     __device__ __forceinline__ uint64_t load(int j) const {
         if (k == 0) return barrett_prod_lazy(mul_wide(a1[j], a2[j]), q, mh);
@@ -447,8 +469,20 @@ struct DecSrc {
     const uint64_t* sk;
     DevConsts dc;
     struct Row {
+        static constexpr bool kLoadAdj = true;
         const uint64_t *a, *b, *s;
         uint64_t q, mh, ml;
+        template <int K>
+        __device__ __forceinline__ void load_adj(int j, uint64_t* x) const {
+            const bool wide = wide_ok(a) && wide_ok(b) && wide_ok(s);
+            uint64_t y[K], z[K];
+            load_adjacent<K>(a + j, wide, x);
+            load_adjacent<K>(s + j, wide, y);
+            load_adjacent<K>(b + j, wide, z);
+#pragma unroll
+            for (int i = 0; i < K; i++)
+                x[i] = csub63(barrett_prod_lazy(mul_wide(x[i], y[i]), q, mh), q << 1) + z[i];
+        }
         // a and s fully reduced: one-high-product Barrett (mh holds its constant); below 3q
         __device__ __forceinline__ uint64_t load(int j) const {
             return csub63(barrett_prod_lazy(mul_wide(a[j], s[j]), q, mh), q << 1) + b[j];
