@@ -411,12 +411,19 @@ static inline MulScratch mul_scratch_layout(const Context& c, int count, uint8_t
     return m;
 }
 // Sub-batches of a batched multiply hold at least Context::min_branch_pairs
-// pairs (default 1; KBFV_TUNE_MIN_BRANCH_PAIRS): from 2 pairs on, two
-// sub-batches on two streams fill the SMs that one batch's launches of fewer
-// rows than SMs leave idle (3 pairs 0.252 -> 0.243 ms against a minimum of 2;
-// 4 pairs 0.314 -> 0.265 ms, 8 pairs 0.481 -> 0.408 ms, 12 pairs 0.679 ->
-// 0.597 ms on the B200 against a minimum of 8).
+// pairs (default 1; KBFV_TUNE_MIN_BRANCH_PAIRS). Two of them on two streams fill
+// the SMs that one batch's launches leave idle, unless the whole batch is a few rows
+// of a small ring: those launches run on clusters, last a few microseconds each and
+// start early behind one another on one stream (ntt_cluster.cuh), and a second
+// sequence of them costs more than its overlap gives. One / two sub-batches, us:
+//   N = 4096, 2 primes: 2 pairs 59 / 73, 10 pairs 89 / 91, 16 pairs 109 / 107, 32 pairs 164 / 148
+//   N = 8192, 3 primes: 2 pairs 70 / 82, 5 pairs 99 / 100, 8 pairs 133 / 119
+//   N = 16384, 7 primes: 2 pairs 122 / 125, 3 pairs 183 / 168, 8 pairs 349 / 326
+//   N = 32768, 14 primes: 2 pairs 466 / 409
+// so up to 80 rows over Q and 2^19 points a batch is one sub-batch.
 static inline int branch_count(const Context& c, int cnt) {
+    const size_t rows = (size_t)4 * c.nq * cnt;
+    if (rows <= 80 && (rows << c.logn) <= (size_t)1 << 19) return 1;
     return std::max(1, std::min(c.branches, cnt / std::max(1, c.min_branch_pairs)));
 }
 static inline size_t branch_region_bytes(const Context& c, int per) {
