@@ -155,17 +155,17 @@ static inline bool cluster_rows(const DevConsts& dc, int rows) {
     }
 }
 template <int LOGN, class Src, class Dst, bool FULL>
-static void launch_fwd_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
+static void launch_fwd_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st, int row0 = 0) {
     using SH = ClusterShape<LOGN>;
     static_assert(SH::SMEM_BYTES <= 48 << 10, "no attribute needed");
     launch_clusters(dc.shape.tail_sms > 0, ntt_fwd_cluster_kernel<LOGN, Src, Dst, FULL>, (unsigned)rows << kClusterLog,
-                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_fwd, dc.mods);
+                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_fwd, dc.mods, row0);
 }
 template <int LOGN, class Src, class Dst>
-static void launch_inv_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st) {
+static void launch_inv_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st, int row0 = 0) {
     using SH = ClusterShape<LOGN>;
     launch_clusters(dc.shape.tail_sms > 0, ntt_inv_cluster_kernel<LOGN, Src, Dst>, (unsigned)rows << kClusterLog,
-                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_inv, dc.mods);
+                    SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_inv, dc.mods, row0);
 }
 
 template <int LOGB, class Src, class Dst, bool FULL = true>
@@ -223,18 +223,28 @@ constexpr int kSplitRows14Default = 48;
 // default of LaunchShape::split_rows_alone (KBFV_TUNE_SPLIT_ROWS_ALONE).
 constexpr int kSplitRowsAloneDefault = 148;
 
-// Whether `rows` transforms of 2^14 points run split. A wave of whole-ring CTAs
-// (one per SM) takes 25 us however few rows it has; the split form takes 12 us plus
-// 0.19 us a row. So up to five waves, a launch that has the GPU to itself runs
-// split while its last wave holds at most 96 - 14 (waves - 1) rows (150 rows: 53
-// us whole, 41 split; 231: 55, 54; 333: 80, 68; 448: 105, 94; 600: 132, 123; but
-// 296: 56, 64 and 370: 80, 76 not split). Beside a sibling sub-batch the last
-// wave's idle SMs are not idle (tail_sms 0).
+// A wave of whole-ring CTAs of 2^14 points (one per SM) takes 25 us however few
+// rows it has. A launch that has the GPU to itself (tail_sms > 0; beside a sibling
+// sub-batch the last wave's idle SMs are not idle) leaves the rows of a short last
+// wave to a launch of clusters behind it: at most one cluster CTA per SM (18 rows,
+// 8-13 us), or 64 rows (17 us) from the fourth wave on, where the other form of a
+// short wave, the split of all rows below, has lost its lead. Us, with / without:
+// forward 150 rows 33 / 39, 310: 57 / 63, 448: 80 / 86, 508: 88 / 95, 600: 104 / 113,
+// 800: 144 / 150, 900: 160 / 170; inverse 150: 34 / 40, 448: 82 / 93, 900: 162 / 183.
+static inline int tail_rows14(const LaunchShape& sh, int rows) {
+    if (sh.tail_sms <= 0 || rows <= sh.split_rows14 || rows <= sh.tail_sms) return 0;
+    const int full = rows / sh.tail_sms, rest = rows % sh.tail_sms;
+    return rest << kClusterLog <= sh.tail_sms || (full >= 3 && rest <= 64) ? rest : 0;
+}
+// Whether `rows` transforms of 2^14 points run split: few rows, or two and three
+// waves of which the last one holds at most 96 - 14 (waves - 1) rows; the split form
+// takes 12 us plus 0.17 us a row (180 rows: 50 us whole, 39 split; 231: 52, 50; 333:
+// 72, 64; but 256: 49, 52 and 370: 72, 71 not split).
 static inline bool split14(const LaunchShape& sh, int rows) {
     if (rows <= sh.split_rows14) return true;
     if (sh.tail_sms <= 0) return false;
     const int waves = (rows + sh.tail_sms - 1) / sh.tail_sms;
-    return waves >= 2 && waves <= 5 && rows - (waves - 1) * sh.tail_sms <= 96 - 14 * (waves - 1);
+    return waves >= 2 && waves <= 3 && rows - (waves - 1) * sh.tail_sms <= 96 - 14 * (waves - 1);
 }
 
 // Forward NTT of `rows` rows read through `s` and written through `d`. Few rows of
@@ -263,6 +273,11 @@ static void ntt_fwd(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st
         case 12: launch_fwd_block<12, Src, Dst, FULL>(dc, s, d, rows, 12, st); break;
         case 13: launch_fwd_block<13, Src, Dst, FULL>(dc, s, d, rows, 13, st); break;
         case 14: {
+            if (const int tail = tail_rows14(dc.shape, rows)) {
+                launch_fwd_block<14, Src, Dst, FULL>(dc, s, d, rows - tail, 14, st);
+                launch_fwd_cluster<14, Src, Dst, FULL>(dc, s, d, tail, st, rows - tail);
+                break;
+            }
             if (!split14(dc.shape, rows)) {
                 launch_fwd_block<14, Src, Dst, FULL>(dc, s, d, rows, 14, st);
                 break;
@@ -314,6 +329,11 @@ static void ntt_inv(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st
         case 12: launch_inv_block<12, Src, Dst, true>(dc, s, d, rows, 12, st); break;
         case 13: launch_inv_block<13, Src, Dst, true>(dc, s, d, rows, 13, st); break;
         case 14: {
+            if (const int tail = tail_rows14(dc.shape, rows)) {
+                launch_inv_block<14, Src, Dst, true>(dc, s, d, rows - tail, 14, st);
+                launch_inv_cluster<14, Src, Dst>(dc, s, d, tail, st, rows - tail);
+                break;
+            }
             if (!split14(dc.shape, rows)) {
                 launch_inv_block<14, Src, Dst, true>(dc, s, d, rows, 14, st);
                 break;

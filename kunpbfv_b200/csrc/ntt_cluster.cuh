@@ -142,12 +142,12 @@ __device__ __forceinline__ void cluster_inv_passes(uint64_t* sm, const tw_t* tw,
 // Forward: outputs as ntt_fwd_block_kernel's (FULL: reduced, else below 8q).
 template <int LOGN, class Src, class Dst, bool FULL = true>
 static __global__ void __launch_bounds__(ClusterShape<LOGN>::THREADS)
-ntt_fwd_cluster_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const uint64_t* __restrict__ mods) {
+ntt_fwd_cluster_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const uint64_t* __restrict__ mods, int row0) {
     constexpr int LOGB = ClusterShape<LOGN>::LOGB, NB = ClusterShape<LOGN>::NB, T = ClusterShape<LOGN>::THREADS;
     extern __shared__ uint64_t sm[];
     cluster_arrive();  // every CTA of the cluster runs before its shared memory is written
     pdl_trigger();
-    const int row = blockIdx.x >> kClusterLog, blk = (int)cluster_rank(), t = threadIdx.x;
+    const int row = row0 + (int)(blockIdx.x >> kClusterLog), blk = (int)cluster_rank(), t = threadIdx.x;
     const RowTab rt = row_tab(src, row, false, tw_all, mods, LOGN);
     const auto s = src.bind(row);
     const uint64_t q = rt.q, q4 = q << 2;
@@ -186,11 +186,11 @@ ntt_fwd_cluster_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const 
 // Inverse: n^-1 applied, fully reduced.
 template <int LOGN, class Src, class Dst>
 static __global__ void __launch_bounds__(ClusterShape<LOGN>::THREADS)
-ntt_inv_cluster_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const uint64_t* __restrict__ mods) {
+ntt_inv_cluster_kernel(Src src, Dst dst, const tw_t* __restrict__ tw_all, const uint64_t* __restrict__ mods, int row0) {
     constexpr int LOGB = ClusterShape<LOGN>::LOGB, NB = ClusterShape<LOGN>::NB, T = ClusterShape<LOGN>::THREADS;
     extern __shared__ uint64_t sm[];
     pdl_trigger();
-    const int row = blockIdx.x >> kClusterLog, blk = (int)cluster_rank(), t = threadIdx.x;
+    const int row = row0 + (int)(blockIdx.x >> kClusterLog), blk = (int)cluster_rank(), t = threadIdx.x;
     const RowTab rt = row_tab(src, row, true, tw_all, mods, LOGN);
     const auto s = src.bind(row);
     const uint64_t q = rt.q, q4 = q << 2;

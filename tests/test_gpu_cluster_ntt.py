@@ -1,5 +1,6 @@
 """Transforms of few rows run with one row over a cluster of CTAs: every ring
-degree that has the form, at one row and on both sides of each limit of the rule, forward against the oracle and back, with no synchronisation between
+degree that has the form, at one row and on both sides of each limit of the rule
+(the rows of a short last wave too, on a GPU of 148 SMs), forward against the oracle and back, with no synchronisation between
 the launches (they start while the one before still runs); and a chain of calls
 whose outputs the next call reads and overwrites at once."""
 import numpy as np
@@ -11,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("log_n,rows", [(12, 1), (12, 128), (12, 129), (13, 1), (13, 128), (13, 129),
-                                        (14, 1), (14, 18), (14, 19), (14, 38), (14, 112), (14, 113), (15, 1), (15, 8), (15, 9)])
+                                        (14, 1), (14, 18), (14, 19), (14, 38), (14, 112), (14, 113), (14, 149), (14, 166), (14, 167),
+                                        (14, 314), (14, 508), (14, 509), (15, 1), (15, 8), (15, 9)])
 def test_few_rows(log_n, rows):
     import oracle
     ps = oracle.primes_bits(1 << log_n, 60, 4)
