@@ -446,10 +446,8 @@ int kbfv_apply_galois(kbfv_context* ctx, const uint64_t* d_gk, uint64_t galois_e
             galois_b_kernel<<<row_blocks<1>((size_t)cnt * c.nq, c.logn), 256, 0, st>>>(in, m.sb, galois_elt, c.logn, c.nq);
             check_launch("galois_b");
             // g(a) read through the permutation by the inverse NTT, then the hybrid key switch
-            ntt_inv(dc, GaloisASrc{in, galois_elt, dc.logn, dc.nq}, digit_rows(dc, m.sd2), cnt * dc.nq, st);
-            lift_launch(dc, m.sd2, cnt, st);
-            ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sd2, 0, dc.npq), rows_io(dc, m.sd2, 0, dc.npq),
-                                          cnt * dc.dnum * dc.npq, st);
+            ntt_inv(dc, GaloisASrc{in, galois_elt, dc.logn, dc.nq}, digit_rows(dc, m), cnt * dc.nq, st);
+            digits_ntt(dc, m, cnt, true, st);
             std::vector<uint64_t*> O(cnt);
             std::vector<const uint64_t*> Z(cnt);
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }

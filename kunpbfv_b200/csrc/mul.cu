@@ -45,6 +45,16 @@ void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int 
     ntt_fwd(dc, ModDownKeySrc{se, add, dc}, OutCtKeyDst{pb, sd2, key, dc, ndig, ex}, count * 2 * dc.nq, st);
 }
 
+void digits_ntt(const DevConsts& dc, const MulScratch& m, int count, bool lift, cudaStream_t st) {
+    const RowsIO rows = rows_io(dc, m.sd2, 0, dc.npq);
+    if (lift_in_ntt(dc)) {
+        ntt_fwd<LiftOneSrc, RowsIO, true>(dc, LiftOneSrc{m.se, dc}, rows, count * dc.dnum * dc.npq, st);
+        return;
+    }
+    if (lift) lift_launch(dc, m.sd2, count, st);
+    ntt_fwd<RowsIO, RowsIO, true>(dc, rows, rows, count * dc.dnum * dc.npq, st);
+}
+
 void mul_front(const DevConsts& dc, const PtrBatch& pb, int count, const MulScratch& m, cudaStream_t st) {
     // K1: INTT over Q of [a1, b1, a2, b2], stored as y_i = [x_i (Q/q_i)^-1]_{q_i}
     ntt_inv(dc, PairQRowsP{pb, dc.logn, dc.nq}, QHatRowsIO{m.sa, dc.logn, dc.nq, dc.q2r_fold}, count * 4 * dc.nq, st);
@@ -69,10 +79,14 @@ void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* ou
 void mul_relin_chunk(const DevConsts& dc, const uint64_t* rlk, const PtrBatch& pb, int count, const MulScratch& m,
                      cudaStream_t st) {
     mul_front(dc, pb, count, m, st);
-    k5_launch(dc, count, m, nullptr, 1, st);
-    // K6a: NTT over Q|P of the lifted digits, in place, fully reduced (key product uses barrett_prod)
-    ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sd2, 0, dc.npq), rows_io(dc, m.sd2, 0, dc.npq),
-                                   count * dc.dnum * dc.npq, st);
+    if (lift_in_ntt(dc)) {
+        MulScratch k5 = m;
+        k5.sd2 = m.se;  // a1 a2's limbs where digit_rows says
+        k5_launch(dc, count, k5, nullptr, 2, st);
+    } else {
+        k5_launch(dc, count, m, nullptr, 1, st);
+    }
+    digits_ntt(dc, m, count, false, st);
     // K6b: key product over P fused into INTT over P; K7: mod down + add (cross |
     // b1b2) fused into NTT over Q, the key product over Q added at its store
     ks_tail(dc, m.sd2, rlk, dc.dnum, m.se, m.sd, pb, count, st);
@@ -132,10 +146,8 @@ int kbfv_relinearize(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_t* d
             const uint64_t* tz = d_tensor + (size_t)off * 3 * lq;
             uint64_t* out = d_ct + (size_t)off * 2 * lq;
             // INTT of a1*a2 (rows (item, limb) of the tensor's first poly) into the digits' own limbs, then the lift
-            ntt_inv(dc, TensorA2{tz, dc.logn, dc.nq}, digit_rows(dc, m.sd2), cnt * dc.nq, st);
-            lift_launch(dc, m.sd2, cnt, st);
-            ntt_fwd<RowsIO, RowsIO, true>(dc, rows_io(dc, m.sd2, 0, dc.npq), rows_io(dc, m.sd2, 0, dc.npq),
-                                           cnt * dc.dnum * dc.npq, st);
+            ntt_inv(dc, TensorA2{tz, dc.logn, dc.nq}, digit_rows(dc, m), cnt * dc.nq, st);
+            digits_ntt(dc, m, cnt, true, st);
             std::vector<uint64_t*> O(cnt);
             std::vector<const uint64_t*> Z(cnt);
             for (int i = 0; i < cnt; i++) { O[i] = out + (size_t)i * 2 * lq; Z[i] = nullptr; }

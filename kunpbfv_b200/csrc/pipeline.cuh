@@ -503,20 +503,75 @@ struct DecSrc {
 };
 
 
-// an inverse transform's rows (item, limb of Q) stored at the digits' own limbs:
-// [item][dnum][Q|P], limb i in digit i / alpha
+// an inverse transform's rows (item, limb of Q) stored at the digits' own limbs
+// ([item][dnum][Q|P], limb i in digit i / alpha), or one after the other
 struct DigitRowsIO {
-    uint64_t* sd2;
-    int logn, nq, npq, dnum, alpha;
+    uint64_t* base;
+    int logn, nq;
+    size_t item, digit;  // strides in rows
+    int alpha;
     __device__ __forceinline__ int prime(int row) const { return row % nq; }
     __device__ __forceinline__ PtrRow bind(int row) const {
-        const int item = row / nq, l = row % nq;
-        return PtrRow{sd2 + ((((size_t)item * dnum + l / alpha) * npq + l) << logn)};
+        const int l = row % nq;
+        return PtrRow{base + (((row / nq) * item + (l / alpha) * digit + l) << logn)};
     }
 };
-static inline DigitRowsIO digit_rows(const DevConsts& dc, uint64_t* sd2) {
-    return DigitRowsIO{sd2, dc.logn, dc.nq, dc.npq, dc.dnum, dc.alpha};
+
+// Digits of one prime each need no lift kernel: a digit's word in the prime of
+// another limb is x, less q_d where the key switch's single-precision quotient
+// estimate x / q_d rounds to 1, and the transform over Q|P takes it as it loads
+// (7 digits of 8 ciphertexts at N = 16384: a 29 us launch and its 59 MB less). The
+// coefficients then stand in se (free until the tail), which the transforms of the
+// digits' own limbs do not overwrite.
+static inline bool lift_in_ntt(const DevConsts& dc) { return dc.alpha == 1 && dc.dnum == dc.nq; }
+// where the digits' coefficient-form limbs go
+static inline DigitRowsIO digit_rows(const DevConsts& dc, const MulScratch& m) {
+    if (lift_in_ntt(dc)) return DigitRowsIO{m.se, dc.logn, dc.nq, (size_t)dc.nq, 0, 1};
+    return DigitRowsIO{m.sd2, dc.logn, dc.nq, (size_t)dc.dnum * dc.npq, (size_t)dc.npq, dc.alpha};
 }
+// smallest x whose single-precision value is that of q (x / q then rounds to 1; below it, to less)
+__device__ __forceinline__ uint64_t float_equal_from(uint64_t q) {
+    const float f = __ull2float_rn(q);
+    const uint64_t hi = (uint64_t)f, lo = (uint64_t)__uint_as_float(__float_as_uint(f) - 1);
+    if (hi - lo < 2) return hi;  // exact below 2^24
+    return ((hi + lo) >> 1) + (__float_as_uint(f) & 1);  // the tie goes to the even one
+}
+struct LiftOneRow {
+    static constexpr bool kLoadMany = true;
+    const uint64_t* x;
+    uint64_t from, less;  // x >= from: plus less = -q_d mod q
+    uint64_t q, mh;       // reduce: x may exceed 4q
+    bool reduce;
+    // below 5q
+    template <int K>
+    __device__ __forceinline__ void load_n(const int (&j)[K], uint64_t* v) const {
+#pragma unroll
+        for (int i = 0; i < K; i++) v[i] = x[j[i]];
+#pragma unroll
+        for (int i = 0; i < K; i++) {
+            const uint64_t add = v[i] >= from ? less : 0;
+            if (reduce) v[i] -= __umul64hi(v[i], mh) * q;
+            v[i] += add;
+        }
+    }
+    __device__ __forceinline__ void store(int, uint64_t) const {}
+};
+struct LiftOneSrc {  // rows (item, digit, limb of Q|P)
+    const uint64_t* x;  // [item][nq], coefficient form
+    DevConsts dc;
+    __device__ __forceinline__ int prime(int row) const { return row % dc.npq; }
+    __device__ __forceinline__ LiftOneRow bind(int row) const {
+        const int m = row % dc.npq, g = row / dc.npq % dc.dnum;
+        const uint64_t qd = dc.mods[g], q = dc.mods[m], mh = dc.mu_hi[m];
+        LiftOneRow r;
+        r.x = x + ((size_t)(row / dc.npq) << dc.logn);  // item * nq + digit
+        r.from = m == g ? ~0ULL : float_equal_from(qd);
+        r.less = q - barrett64(qd, q, mh);
+        r.q = q; r.mh = mh;
+        r.reduce = (qd >> 2) > q;
+        return r;
+    }
+};
 
 // INTT over Q of the four input polynomials, Q -> R, NTT over R, fused tensor +
 // INTT over Q|R: steps shared by kbfv_mul and the fused multiply-relinearise.
@@ -532,6 +587,9 @@ void k5_launch_m(const DevConsts& dc, int count, const MulScratch& m, uint64_t* 
 void k5_launch(const DevConsts& dc, int count, const MulScratch& m, uint64_t* out0, int mode, cudaStream_t st);
 // the key-switch lift of the digits' own limbs in sd2 ([item][dnum][npq]) into every other prime of Q|P (lift.cu)
 void lift_launch(const DevConsts& dc, uint64_t* sd2, int count, cudaStream_t st);
+// K6a: the digits' limbs (digit_rows) lifted and transformed over Q|P, into sd2
+// ([item][dnum][npq]), fully reduced; `lift`: the lift is still to do
+void digits_ntt(const DevConsts& dc, const MulScratch& m, int count, bool lift, cudaStream_t st);
 // key-switch tail: key product, mod down and add, written to the outputs of pb
 void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int ndig, uint64_t* se,
              const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st, const KsExtra& ex = {});

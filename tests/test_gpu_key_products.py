@@ -69,3 +69,37 @@ def test_rotation_and_level():
     sq = host(sch.mult_relin(c7, c7).cipher_device).reshape(5, 2, 7, ctx.N)
     for i in (0, 4):
         assert np.array_equal(sq[i], o7.mul_relin(h7[i], h7[i], rl)), i
+
+
+@pytest.mark.parametrize("log_n,q_bits,p_bits", [(10, [50], 52), (12, [60, 60, 60], 60), (13, [60, 36, 60, 36], 60),
+                                                 (14, [36, 60], 36), (15, [30, 59, 45], 60)])
+def test_one_prime_digits_near_the_modulus(log_n, q_bits, p_bits):
+    """Digits of one prime whose coefficients lie where the single-precision
+    quotient x / q rounds to 1 or just does not, over primes of unequal sizes."""
+    import oracle
+    pool = {b: oracle.primes_bits(1 << log_n, b, 5) for b in set(q_bits) | {p_bits}}
+    qs = [pool[b].pop() for b in q_bits]
+    p = [pool[p_bits].pop()]
+    nq = len(qs)
+    ctx, orc = make_pair(log_n, qs, p, nq)
+    n, npq = ctx.N, nq + 1
+    rlk = rand_rows(orc, list(range(npq)) * 2 * nq, n, 1).reshape(nq, 2, npq, n)
+    d = rand_rows(orc, list(range(nq)) * 3 * 2, n, 2).reshape(2, 3, nq, n)
+    for l, q in enumerate(qs):
+        near = [q - 1 - i for i in range(8)]
+        for s in (22, 23, 24, 25, 26):
+            near += [q - 1 - (q >> s) + i for i in range(-2, 3)]
+        # every midpoint between singles near q, and its neighbours
+        f = np.float32(q)
+        for _ in range(3):
+            g = np.nextafter(f, np.float32(0))
+            mid = (int(f) + int(g)) // 2
+            near += [mid + i for i in (-1, 0, 1)]
+            f = g
+        near = np.array([v for v in near if 0 <= v < q], dtype=np.uint64)
+        x = d[0, 0, l].copy()
+        x[:len(near)] = near
+        d[0, 0, l] = orc.ntt_fwd(l, x)
+    got = _relinearize(ctx, rlk, d)
+    for i in range(2):
+        assert np.array_equal(got[i], orc.relinearize(d[i], rlk)), i
