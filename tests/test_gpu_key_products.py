@@ -103,3 +103,46 @@ def test_one_prime_digits_near_the_modulus(log_n, q_bits, p_bits):
     got = _relinearize(ctx, rlk, d)
     for i in range(2):
         assert np.array_equal(got[i], orc.relinearize(d[i], rlk)), i
+
+
+def test_t_base_blocks_of_one_prime_near_the_modulus():
+    """The T-base key switch whose blocks are one prime each (lifted by the
+    transform's loads) equals its pieces called one by one (lifted by the block
+    kernel), on coefficients where the quotient estimate is 1 or just not."""
+    import torch
+    import kunpbfv_b200 as kb
+    from kunpbfv_b200.api import _check, _ptr, _stream_ptr, lib
+    ctx = kb.reference_context(15)
+    assert ctx.p_count == 1
+    n, nq, nt = ctx.N, ctx.q_count, ctx.t_count
+    nri, nqj, words = ctx.klss_info()
+    rng = np.random.default_rng(8)
+    count = 2
+    x = np.stack([np.stack([rng.integers(0, q, size=n, dtype=np.uint64) for q in ctx.q]) for _ in range(count)])
+    for l, q in enumerate(ctx.q):
+        near = [q - 1 - i for i in range(8)] + [q - 1 - (q >> s) + i for s in (22, 23, 24, 25, 26) for i in range(-2, 3)]
+        f = np.float32(q)
+        for _ in range(3):
+            g = np.nextafter(f, np.float32(0))
+            near += [v for v in ((int(f) + int(g)) // 2 + i for i in (-1, 0, 1)) if v < q]
+            f = g
+        x[0, l, :len(near)] = np.array(near, dtype=np.uint64)
+    key = torch.stack([dev(rng.integers(0, int(ctx.tk[r % nt]), size=n, dtype=np.uint64)) for r in range(words // n)])
+    dig = ctx.klss_modup_qj_to_t(dev(x))
+    ctx.ntt_fwd(dig, ctx.idx_t, nt)
+    z = host(ctx.klss_t_to_pq(ctx.klss_external_product(dig, key))).reshape(count, 2, nq + 1, n)
+    want = np.empty((count, 2, nq, n), dtype=np.uint64)
+    p = int(ctx.p[0])
+    for l, q in enumerate(ctx.q):
+        inv = pow(p, -1, int(q))
+        diff = (z[:, :, l].astype(object) - z[:, :, nq].astype(object)) * inv % int(q)
+        want[:, :, l] = diff.astype(np.uint64)
+    wd = dev(want)
+    ctx.ntt_fwd(wd, 0, nq)
+    d = np.zeros((count, 3, nq, n), dtype=np.uint64)
+    d[:, 0] = x
+    dd = dev(d)
+    ctx.ntt_fwd(dd, 0, nq)
+    out = torch.full((count, 2, nq, n), -1, dtype=torch.int64, device="cuda")
+    _check(lib().kbfv_relinearize_klss(ctx.handle, _ptr(key), _ptr(dd), _ptr(out), count, _stream_ptr(None)))
+    assert np.array_equal(host(out).reshape(want.shape), host(wd).reshape(want.shape))
