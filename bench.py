@@ -561,9 +561,10 @@ def c4_uneven(stream):
 
 
 def step_roofline(ms_step, hbm_peak, peak_kind):
-    """The headline step against the IMAD bound: every primitive of the 9-kernel
-    pipeline counted per pair (kunpbfv_b200.roofline.pipeline_counts), each at
-    the rate kbfv_probe_arith measures for it live on this GPU; and, from the
+    """The headline step against its arithmetic bound: every primitive of the
+    pipeline counted per pair (kunpbfv_b200.roofline.pipeline_counts), those on the
+    IMAD pipe at the rates kbfv_probe_arith measures live on this GPU, the base
+    conversions' byte products at the tensor cores' (step_floor_s); and, from the
     committed ncu summary of the same kernel sources, the IMAD-pipe instructions
     per pair against the measured IMAD issue rate. Beside them the step's HBM
     rate (inputs, outputs and the key read once per launch)."""
@@ -571,14 +572,14 @@ def step_roofline(ms_step, hbm_peak, peak_kind):
     from kunpbfv_b200.api import probe_arith
     pc = rl.pipeline_counts(1 << LOG_N, LOG_N, NQ, NP, 1)
     rates = {k: probe_arith(kind) * 1e9 for k, kind in rl.PROBE_KIND.items()}
-    floor_s = rl.arithmetic_floor_s(pc["counts"], rates)
+    floor_s = rl.step_floor_s(pc, rates)
     step_s = ms_step / 1e3
     n = 1 << LOG_N
     bytes_pair = 4 * NQ * n * 8 + 2 * NQ * n * 8 + 2 * (NQ + NP) * n * 8 // BATCH
     out = {"bound": "imad", "unit": "modmul/s",
            "modmuls_per_pair": pc["products"],
            "reductions_per_pair": pc["counts"]["b128"],
-           "counts_per_pair": pc["counts"], "ntt_rows_per_pair": pc["ntt_rows"], "formula": pc["formula"],
+           "counts_per_pair": pc["counts"], "on_tensor_cores_per_pair": pc["conversions"], "ntt_rows_per_pair": pc["ntt_rows"], "formula": pc["formula"],
            "achieved": round(pc["products"] * BATCH / step_s, 0),
            "peak": round(pc["products"] / floor_s, 0),
            "frac": round(floor_s * BATCH / step_s, 4),

@@ -208,18 +208,16 @@ static void launch_inv_block(const DevConsts& dc, Src s, Dst d, int rows, int lo
 template <class Dst>
 static inline Dst plain_of(const Dst& d) { return d; }
 
-// At N = 2^14, launches of at most this many rows (fewer 1024-thread CTAs
-// than SMs, e.g. one ciphertext pair per call: 2-45 rows) run as a radix-4
-// column pass and 2^12-point blocks: four times the CTAs cover the SMs, 15-23 us
-// instead of 29-31 us per launch of 8-45 rows on the B200. At 64 rows the
-// split alone is still faster, but beside a concurrent sub-batch it cost the
+// At N = 2^14, launches of at most this many rows that do not run on clusters
+// (cluster_rows) run as a radix-4 column pass and 2^12-point blocks: four times the
+// CTAs cover the SMs, 12-17 us instead of 25 us for 19-45 rows on the B200. At 64
+// rows the split alone is still faster, but beside a concurrent sub-batch it cost the
 // batched multiply ~1%, so 64-row launches keep the whole-ring blocks. The
 // default of LaunchShape::split_rows14 (KBFV_TUNE_SPLIT_ROWS).
 constexpr int kSplitRows14Default = 48;
 // The same threshold for a multiply that runs as one stream (batches below two
-// sub-batches, the tensor-only multiply): launches of up to 148 rows would
-// leave SMs idle with one 1024-thread CTA per row, and no sibling sub-batch
-// fills them, so they split (2 pairs: 0.211 -> 0.192 ms on the B200). The
+// sub-batches, the tensor-only multiply), where no sibling sub-batch fills the SMs
+// that few whole-ring CTAs leave idle. The
 // default of LaunchShape::split_rows_alone (KBFV_TUNE_SPLIT_ROWS_ALONE).
 constexpr int kSplitRowsAloneDefault = 148;
 
@@ -248,8 +246,8 @@ static inline bool split14(const LaunchShape& sh, int rows) {
 }
 
 // Forward NTT of `rows` rows read through `s` and written through `d`. Few rows of
-// 2^12..2^15 points run on clusters (cluster_rows). Else, for logn <= 14 one block kernel (N = 2^14 with at most shape.split_rows14 rows:
-// as for 15/16 with a radix-4 column pass); for 15/16 a radix-8/16 column pass
+// 2^12..2^15 points run on clusters (cluster_rows). Else, for logn <= 14 one block
+// kernel (N = 2^14: or as tail_rows14 and split14 say); for 15/16 a radix-8/16 column pass
 // (s -> plain_of(d)) then 2^12-point block kernels from plain_of(d) to d in
 // place (d must also be readable): several 256-thread CTAs per SM run faster
 // than one 1024-thread CTA per 2^14-point block. FULL = false leaves outputs in [0, 8q) for consumers that reduce

@@ -1,6 +1,6 @@
 // Captured multiplies (kbfv_plan_*): a caller that multiplies the same device
 // buffers again and again (a request loop with fixed staging buffers) replays
-// the whole multiply as one CUDA graph launch instead of issuing its ~14
+// the whole multiply as one CUDA graph launch instead of issuing its 8 to 12
 // kernel launches one by one; a batch of pairs at mixed levels
 // (kbfv_mul_relin_levels) likewise becomes one graph launch. No counterpart in
 // the reference.

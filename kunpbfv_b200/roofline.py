@@ -1,8 +1,8 @@
 """Arithmetic roofline of the fused multiply + relinearise pipeline.
 
-At 60-bit moduli every kernel of the multiply is bound by the issue rate of
-64-bit integer multiplies on the IMAD ("fmaheavy") pipe, not by HBM. This
-module counts the modular arithmetic one ciphertext pair costs in the 9-kernel
+At 60-bit moduli the transforms of the multiply, most of its time, are bound by
+the issue rate of 64-bit integer multiplies on the IMAD ("fmaheavy") pipe, not by
+HBM. This module counts the modular arithmetic one ciphertext pair costs in the
 pipeline (kunpbfv_b200/csrc/mul.cu, k5_kernels.cuh, pipeline.cuh), by class of
 primitive:
 
@@ -19,7 +19,11 @@ primitive:
 and turns the counts into the time the step would take if every primitive ran
 at the rate `kbfv_probe_arith` measures for it in register chains on the same
 GPU (no memory traffic, no synchronisation): the arithmetic floor of the step.
-The step's roofline fraction is that floor divided by the measured step time.
+The base conversions' sums and reductions are left out of the step's floor
+(step_floor_s): they run as byte products on the tensor cores (csrc/limb_mma.cuh),
+64 int8 multiply-accumulates for each 64-bit one, a separate pipe whose time is the
+floor only if it is longer. The step's roofline fraction is the floor divided by
+the measured step time.
 
 It also reads the IMAD-pipe instruction counts of the same pipeline from a
 committed ncu summary (profiles/mult_relin_imad_n16384.md) when that summary was
@@ -34,6 +38,9 @@ import re
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
+
+# int8 mma.sync multiply-accumulates per second on a B200 (m16n8k32 u8, register chains)
+IMMA_MACS = 5.7e14
 
 # probe kinds of kbfv_probe_arith measuring each class
 PROBE_KIND = {"bfly": 11, "mac": 10, "prod": 6, "b128": 5, "shoup": 4}
@@ -98,12 +105,21 @@ def pipeline_counts(n: int, log_n: int, nq: int, np_: int, dnum: int) -> dict:
         f" q={nq} r={nr} p={np_} dnum={dnum} N={n}"
     )
     products = c["bfly"] + c["mac"] + c["prod"] + c["shoup"]
-    return {"counts": c, "ntt_rows": ntt_rows, "products": products, "formula": formula}
+    conversions = {"mac": n * (4 * nq * nr + 3 * nr * (nq + 1) + 3 * nr * nq + sum((npq - a) * a for a in digits)),
+                   "b128": n * (4 * nr + 3 * nr + 3 * nq + sum(npq - a for a in digits))}
+    return {"counts": c, "conversions": conversions, "ntt_rows": ntt_rows, "products": products, "formula": formula}
 
 
 def arithmetic_floor_s(counts: dict, rates: dict) -> float:
     """Seconds per pair if every primitive ran at its measured rate (rates in op/s)."""
     return sum(counts[k] / rates[k] for k in counts if counts[k])
+
+
+def step_floor_s(pc: dict, rates: dict) -> float:
+    """Seconds per pair of the pipeline's arithmetic: the IMAD classes without the
+    base conversions, or the conversions' byte products if those take longer."""
+    imad = {k: v - pc["conversions"].get(k, 0) for k, v in pc["counts"].items()}
+    return max(arithmetic_floor_s(imad, rates), 64 * pc["conversions"]["mac"] / IMMA_MACS)
 
 
 def source_sha16(files) -> str:
