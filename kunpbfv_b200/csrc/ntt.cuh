@@ -138,9 +138,13 @@ __device__ __forceinline__ void load_points(const Row& s, uint64_t* x, Index ind
     }
 }
 
-// asynchronous copy of `bytes` (a multiple of 16, 16-byte aligned) into L2
+// Asynchronous copy of `bytes` (a multiple of 16) into L2. The bulk prefetch takes
+// 16-byte aligned addresses only and a caller's rows may be aligned to a word: the
+// range then starts at the 16-byte granule of the first word and the last word is
+// left to the load.
 __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)15;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(bytes) : "memory");
 }
 
 // the block `ahead` CTAs after this one (ahead = CTAs resident at once; 0: none)
