@@ -123,9 +123,12 @@ int kbfv_mul(kbfv_context* ctx, const uint64_t* d_ct1, const uint64_t* d_ct2, ui
             uint64_t* out = d_tensor + (size_t)off * 3 * lq;
             const DevConsts dc = alone_consts(c);  // one stream: no sibling sub-batch fills the SMs
             mul_front(dc, pb, cnt, m, st);
-            k5_launch(dc, cnt, m, out, 0, st);
-            RowsIO io = rows_io(dc, out, 0, c.nq);
-            ntt_fwd(dc, io, io, cnt * 3 * c.nq, st);
+            // K5 stores 16 bytes at a time: a tensor aligned to a word only is stored
+            // to sa (4 nq limbs a pair, dead since K2), the transform, whose stores are
+            // words, moves it
+            uint64_t* coef = aligned16({out}) ? out : m.sa;
+            k5_launch(dc, cnt, m, coef, 0, st);
+            ntt_fwd(dc, rows_io(dc, coef, 0, c.nq), rows_io(dc, out, 0, c.nq), cnt * 3 * c.nq, st);
         }
     });
 }

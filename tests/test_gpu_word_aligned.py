@@ -54,3 +54,22 @@ def test_encode_decode(log_n, rows, src, dst):
         _check(call(h, px, po, rows, 0))
         assert torch.equal(bo[dst:dst + x.numel()], want)
         assert torch.equal(bx[src:src + x.numel()], x.view(-1)), "the input is not written"
+
+
+# few rows (clusters, split and whole rows) and more than are resident at once
+@pytest.mark.parametrize("log_n,pairs", [(10, 1), (12, 1), (12, 130), (13, 4), (14, 1), (14, 60), (15, 1), (15, 30),
+                                         (16, 1)])
+def test_tensor(log_n, pairs):
+    """kbfv_mul with its inputs and its tensor word-aligned, each alone and both"""
+    from kunpbfv_b200.api import _check, lib
+    ctx, _ = small_pair(log_n=log_n, nq=2, np_=1, bits=50)
+    L, h = lib(), ctx.handle
+    a, b = (_words((pairs, 2, 2, ctx.N), min(ctx.q), s) for s in (3, 4))
+    want = torch.empty(pairs * 3 * 2 * ctx.N, dtype=torch.int64, device="cuda")
+    _check(L.kbfv_mul(h, a.data_ptr(), b.data_ptr(), want.data_ptr(), pairs, 0))
+    for src, dst in ((0, 1), (1, 0), (1, 1)):
+        (ba, pa), (bb, pb) = _put(a, src), _put(b, src)
+        bo, po = _put(torch.zeros_like(want), dst)
+        _check(L.kbfv_mul(h, pa, pb, po, pairs, 0))
+        assert torch.equal(bo[dst:dst + want.numel()], want), (src, dst)
+        assert not bo[:dst].any() and not bo[dst + want.numel():].any(), "nothing is written beside the tensor"
