@@ -111,6 +111,19 @@ static inline int resident_ctas_at(const void* kernel, int threads, int smem, in
     return cache[i];
 }
 
+// Allows `kernel` up to `bytes` of dynamic shared memory (without it a launch may
+// take 48 KB). The permission belongs to the kernel in one CUDA context, so it is
+// asked for at each launch (53 ns) instead of remembered per process, where another
+// GPU's context would go without; and always for the same value, the kernel's
+// largest at any CTA size, so that threads with different CTA sizes do not lower it
+// for one another.
+constexpr int kPlainSmem = 48 << 10;
+template <class K>
+static inline void allow_smem(K kernel, int bytes) {
+    if (bytes > kPlainSmem)
+        KB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
 // A launch of clusters of `cluster` CTAs. `early`: it may start while the kernel
 // before it on the stream still runs (programmatic dependent launch; the kernel
 // waits before it touches memory that other kernels use).
@@ -157,7 +170,7 @@ static inline bool cluster_rows(const DevConsts& dc, int rows) {
 template <int LOGN, class Src, class Dst, bool FULL>
 static void launch_fwd_cluster(const DevConsts& dc, Src s, Dst d, int rows, cudaStream_t st, int row0 = 0) {
     using SH = ClusterShape<LOGN>;
-    static_assert(SH::SMEM_BYTES <= 48 << 10, "no attribute needed");
+    static_assert(SH::SMEM_BYTES <= kPlainSmem, "no permission needed");
     launch_clusters(dc.shape.tail_sms > 0, ntt_fwd_cluster_kernel<LOGN, Src, Dst, FULL>, (unsigned)rows << kClusterLog,
                     SH::THREADS, SH::SMEM_BYTES, 1u << kClusterLog, st, s, d, dc.tw_fwd, dc.mods, row0);
 }
@@ -171,15 +184,10 @@ static void launch_inv_cluster(const DevConsts& dc, Src s, Dst d, int rows, cuda
 template <int LOGB, class Src, class Dst, bool FULL = true>
 static void launch_fwd_block(const DevConsts& dc, Src s, Dst d, int rows, int logn, cudaStream_t st) {
     constexpr int SMEM = BlockShape<LOGB>::SMEM_BYTES;
-    static bool configured = false;
-    static int resident = 0;  // CTAs of this kernel resident at once on the device
-    if (!configured) {
-        KB_CHECK_CUDA(cudaFuncSetAttribute(ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        resident = resident_ctas((const void*)ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>,
-                                 BlockShape<LOGB>::THREADS, SMEM);
-        configured = true;
-    }
+    allow_smem(ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>, SMEM);
+    // CTAs of this kernel resident at once on the device
+    static const int resident = resident_ctas((const void*)ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>,
+                                              BlockShape<LOGB>::THREADS, SMEM);
     const int nblk = 1 << (logn - LOGB);
     ntt_fwd_block_kernel<LOGB, Src, Dst, FULL><<<rows * nblk, BlockShape<LOGB>::THREADS, SMEM, st>>>(
         s, d, dc.tw_fwd, dc.mods, logn, dc.shape.l2_prefetch ? resident : 0);
@@ -188,15 +196,10 @@ static void launch_fwd_block(const DevConsts& dc, Src s, Dst d, int rows, int lo
 template <int LOGB, class Src, class Dst, bool WHOLE>
 static void launch_inv_block(const DevConsts& dc, Src s, Dst d, int rows, int logn, cudaStream_t st) {
     constexpr int SMEM = BlockShape<LOGB>::SMEM_BYTES;
-    static bool configured = false;
-    static int resident = 0;  // CTAs of this kernel resident at once on the device
-    if (!configured) {
-        KB_CHECK_CUDA(cudaFuncSetAttribute(ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        resident = resident_ctas((const void*)ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>,
-                                 BlockShape<LOGB>::THREADS, SMEM);
-        configured = true;
-    }
+    allow_smem(ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>, SMEM);
+    // CTAs of this kernel resident at once on the device
+    static const int resident = resident_ctas((const void*)ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>,
+                                              BlockShape<LOGB>::THREADS, SMEM);
     const int nblk = 1 << (logn - LOGB);
     ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE><<<rows * nblk, BlockShape<LOGB>::THREADS, SMEM, st>>>(
         s, d, dc.tw_inv, dc.mods, logn, dc.shape.l2_prefetch ? resident : 0);

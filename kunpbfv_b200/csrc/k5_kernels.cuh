@@ -246,14 +246,12 @@ static __global__ void __maxnreg__(KS <= 4 && !PREP ? 80 : 128) ext_mma_kernel(J
 template <int KS, int NG, bool EXTRA, bool PREP, bool SH, class Job>
 static void ext_mma_launch_sh(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
     static int res[4] = {0, 0, 0, 0};
-    const int smem = mma_stage_bytes(KS + (EXTRA ? 1 : 0), NG) + 4 * KS * 8 +
-                     threads / 32 * 2 * 4 * KS * kRow<mma_tiles(KS)> * 8;
-    static int allowed = 48 << 10;  // dynamic shared memory of a launch without an attribute
-    if (smem > allowed) {
-        KB_CHECK_CUDA(cudaFuncSetAttribute(ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        allowed = smem;
-    }
+    auto smem_of = [](int threads) {
+        return mma_stage_bytes(KS + (EXTRA ? 1 : 0), NG) + 4 * KS * 8 +
+               threads / 32 * 2 * 4 * KS * kRow<mma_tiles(KS)> * 8;
+    };
+    const int smem = smem_of(threads);
+    allow_smem(ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, smem_of(512));
     const int each = threads / 2 * mma_tiles(KS);
     const int iters = mma_iters(polys, logn, each,
                                 resident_ctas_at((const void*)ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, threads, smem, res));
@@ -590,15 +588,13 @@ static __global__ void __launch_bounds__(256, KS <= 4 ? 3 : 1) k5_mma_kernel(Job
 template <int KS, int NG, bool FUSED, bool SH, class Job>
 static void k5_mma_launch_sh(const Job& job, int polys, int logn, int threads, cudaStream_t st) {
     static int res[4] = {0, 0, 0, 0};
-    const int smem = mma_stage_bytes(KS, NG) + mma_stage_bytes(2 * NG + 1, NG) + 4 * (KS + 2 * NG) * 8 +
-                     threads / 32 * 2 * 4 * (KS + 2 * NG) * kRow<mma_tiles(KS)> * 8;
+    auto smem_of = [](int threads) {
+        return mma_stage_bytes(KS, NG) + mma_stage_bytes(2 * NG + 1, NG) + 4 * (KS + 2 * NG) * 8 +
+               threads / 32 * 2 * 4 * (KS + 2 * NG) * kRow<mma_tiles(KS)> * 8;
+    };
+    const int smem = smem_of(threads);
     const int each = threads / 2 * mma_tiles(KS);
-    static int allowed = 48 << 10;  // dynamic shared memory of a launch without an attribute
-    if (smem > allowed) {
-        KB_CHECK_CUDA(cudaFuncSetAttribute(k5_mma_kernel<KS, NG, FUSED, SH, Job>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        allowed = smem;
-    }
+    allow_smem(k5_mma_kernel<KS, NG, FUSED, SH, Job>, smem_of(256));
     const int iters = mma_iters(polys, logn, each,
                                 resident_ctas_at((const void*)k5_mma_kernel<KS, NG, FUSED, SH, Job>, threads, smem, res));
     k5_mma_kernel<KS, NG, FUSED, SH, Job><<<mma_blocks(polys, logn, each, iters), threads, smem, st>>>(job, logn, iters);
