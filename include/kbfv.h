@@ -255,7 +255,10 @@ int kbfv_mul_relin_batch(kbfv_context* ctx, const uint64_t* d_rlk, const uint64_
  * auxiliary streams of the context, forked from and joined back into the
  * caller's stream with events (the call stays ordered on `stream`); the partial
  * last wave of one sub-batch's kernels then overlaps the others'. branches: 1..4
- * sub-batches (default 2; 1 disables). No counterpart in the reference. */
+ * sub-batches (default 2; 1 disables). Until the caller chooses, with this call
+ * or one of the knobs KBFV_TUNE_BRANCHES and KBFV_TUNE_MIN_BRANCH_PAIRS, a batch
+ * of at most 80 rows over Q (4 x q_count a pair) and 2^19 points is not cut: it is
+ * faster whole. No counterpart in the reference. */
 int kbfv_set_branches(kbfv_context* ctx, uint32_t branches);
 /* ---- tuning ---------------------------------------------------------------
  * Per-context knobs that change speed only, never results. The Python module
@@ -266,7 +269,8 @@ typedef enum {
     KBFV_TUNE_NTT_BLOCK_LOG = 0, /* 0 (default: built-in shapes) or 12..14: kbfv_ntt_fwd/inv on
                                     rings above 2^v points run as a column pass of log_n - v
                                     stages and blocks of 2^v points */
-    KBFV_TUNE_BRANCHES = 1,      /* 1..4 (default 2): sub-batches of a batched multiply */
+    KBFV_TUNE_BRANCHES = 1,      /* 1..4 (default 2): sub-batches of a batched multiply
+                                    (kbfv_set_branches, also for the smallest batches) */
     KBFV_TUNE_HOST_CHUNK = 2,    /* 0..128 (default 0 = ~32 MiB of inputs): pairs per chunk of
                                     kbfv_mul_relin_host when its chunk_pairs is 0 */
     KBFV_TUNE_SPLIT_ROWS = 3,    /* 0..2^20 (default 48): at N = 2^14, transforms of at most this
@@ -296,7 +300,8 @@ typedef enum {
                                     kbfv_mul), where no sibling sub-batch fills idle SMs */
     KBFV_TUNE_MIN_BRANCH_PAIRS = 11 /* 1..64 (default 1): a batched multiply splits into
                                     KBFV_TUNE_BRANCHES sub-batches only with at least this many
-                                    pairs in each */
+                                    pairs in each (kbfv_set_branches, also for the smallest
+                                    batches) */
 } kbfv_tune_knob;
 int kbfv_tune_set(kbfv_context* ctx, int knob, int64_t value);
 int kbfv_tune_get(const kbfv_context* ctx, int knob, int64_t* value);

@@ -799,6 +799,7 @@ int kbfv_tune_set(kbfv_context* ctx, int knob, int64_t value) {
             case KBFV_TUNE_BRANCHES:
                 KB_REQUIRE(value >= 1 && value <= 4, KBFV_ERR_INVALID, "branches must be 1..4");
                 c.branches = (int)value;
+                c.branches_chosen = true;
                 break;
             case KBFV_TUNE_HOST_CHUNK:
                 KB_REQUIRE(value >= 0 && value <= kMaxBatch, KBFV_ERR_INVALID, "host chunk must be 0..128");
@@ -841,6 +842,7 @@ int kbfv_tune_set(kbfv_context* ctx, int knob, int64_t value) {
             case KBFV_TUNE_MIN_BRANCH_PAIRS:
                 KB_REQUIRE(value >= 1 && value <= 64, KBFV_ERR_INVALID, "pairs per sub-batch must be 1..64");
                 c.min_branch_pairs = (int)value;
+                c.branches_chosen = true;
                 break;
             default: throw KbfvError(KBFV_ERR_INVALID, "unknown tuning knob");
         }
@@ -851,6 +853,7 @@ int kbfv_tune_set(kbfv_context* ctx, int knob, int64_t value) {
             l.dc.shape = c.dc.shape;
             l.branches = c.branches;
             l.min_branch_pairs = c.min_branch_pairs;
+            l.branches_chosen = c.branches_chosen;
         }
     });
 }
@@ -882,6 +885,7 @@ int kbfv_set_branches(kbfv_context* ctx, uint32_t branches) {
         Context& c = CX(ctx);
         KB_REQUIRE(branches >= 1 && branches <= 4, KBFV_ERR_INVALID, "branches must be 1..4");
         c.branches = (int)branches;
+        c.branches_chosen = true;
     });
 }
 

@@ -146,6 +146,7 @@ struct Context {
     // partial last wave overlaps the others' kernels
     int branches = 2;
     int min_branch_pairs = 1;  // pairs per sub-batch at least (smaller batches run as one stream)
+    bool branches_chosen = false;  // the caller has set one of the two (see branch_count)
     // tuning knobs (kbfv_tune_set): block size 2^ntt_block_log of the standalone
     // NTT on rings above it (the rest runs as a column pass of logn - ntt_block_log
     // stages); pairs per chunk of the host-memory multiply (0: by bytes)

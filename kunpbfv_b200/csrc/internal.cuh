@@ -441,10 +441,11 @@ static inline MulScratch mul_scratch_layout(const Context& c, int count, uint8_t
 //   N = 8192, 3 primes: 2 pairs 70 / 82, 5 pairs 99 / 100, 8 pairs 133 / 119
 //   N = 16384, 7 primes: 2 pairs 122 / 125, 3 pairs 183 / 168, 8 pairs 349 / 326
 //   N = 32768, 14 primes: 2 pairs 466 / 409
-// so up to 80 rows over Q and 2^19 points a batch is one sub-batch.
+// so up to 80 rows over Q and 2^19 points a batch is one sub-batch, until the caller
+// chooses a number of sub-batches or their least size.
 static inline int branch_count(const Context& c, int cnt) {
     const size_t rows = (size_t)4 * c.nq * cnt;
-    if (rows <= 80 && (rows << c.logn) <= (size_t)1 << 19) return 1;
+    if (!c.branches_chosen && rows <= 80 && (rows << c.logn) <= (size_t)1 << 19) return 1;
     return std::max(1, std::min(c.branches, cnt / std::max(1, c.min_branch_pairs)));
 }
 static inline size_t branch_region_bytes(const Context& c, int per) {

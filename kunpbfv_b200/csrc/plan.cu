@@ -27,6 +27,7 @@ struct kbfv_plan {
     void* scratch = nullptr;
     LaunchShape shape{};
     int branches = 0, min_branch_pairs = 0;
+    bool branches_chosen = false;
     uint64_t launches = 0, captures = 0;
 };
 
@@ -42,6 +43,7 @@ void drop_graph(kbfv_plan& p) {
 bool graph_current(const kbfv_plan& p) {
     const Context& c = p.ctx->c;
     return p.exec && c.scratch == p.scratch && c.branches == p.branches && c.min_branch_pairs == p.min_branch_pairs &&
+           c.branches_chosen == p.branches_chosen &&
            std::memcmp(&c.dc.shape, &p.shape, sizeof(LaunchShape)) == 0;
 }
 
@@ -78,6 +80,7 @@ void run_and_capture(kbfv_plan& p, cudaStream_t st) {
     p.shape = c.dc.shape;
     p.branches = c.branches;
     p.min_branch_pairs = c.min_branch_pairs;
+    p.branches_chosen = c.branches_chosen;
     p.captures++;
 }
 
