@@ -46,15 +46,16 @@ HOST_CHUNKS = (4, 8, 12, 16, 24)
 PIPELINE_KNOBS = {
     "branches": (2, 1, 3, 4),
     "bconv_threads": (256, 128, 512, 64),
-    "bconv_cpt": (2, 1),
     "k5_threads": (128, 64, 256),
     "split_rows": (48, 0, 256, 1 << 20),
     "l2_prefetch": (1, 0),
 }
 # tuned on a two-pair multiply (the per-call size it governs)
 K5_FUSED_PAIRS = (2, 0, 4)
-# tuned on one-pair and two-pair multiplies together
-FUSE_Q2R_PAIRS = (1, 0, 2)
+# tuned on the standalone base conversion of the batch's polynomials
+BCONV_CPT = (2, 1)
+# without effect (include/kbfv.h): no candidates to time, the result states the value in force
+FUSE_Q2R_PAIRS = ()
 # tuned on four-pair and eight-pair multiplies (1 and 2 tie there; 1 is 3.5%
 # faster at three pairs)
 MIN_BRANCH_PAIRS = (1, 2, 4, 8)
@@ -204,15 +205,15 @@ def _sweep(ctx, knob, values, run, out, want, reps):
 
 def tune_pipeline(scheme, pairs: int = 64, reps: int = 5) -> Dict[str, object]:
     """The multiply pipeline's knobs (PIPELINE_KNOBS on a batch of `pairs`,
-    K5_FUSED_PAIRS on two pairs, FUSE_Q2R_PAIRS on one and two pairs), one at
-    a time from the defaults; every candidate's product is compared with the
-    default shapes' product."""
+    K5_FUSED_PAIRS on two pairs, BCONV_CPT on a standalone conversion, MIN_BRANCH_PAIRS
+    and SPLIT_ROWS_ALONE on small batches), one at a time from the defaults; every
+    candidate's output is compared with the default shapes' output."""
     import torch
 
     from .api import Ciphertext
     ctx = scheme.context
-    keep = {k: ctx.tune_get(k) for k in list(PIPELINE_KNOBS) + ["k5_fused_pairs", "fuse_q2r_pairs",
-                                                                  "split_rows_alone", "min_branch_pairs"]}
+    keep = {k: ctx.tune_get(k) for k in list(PIPELINE_KNOBS) + ["k5_fused_pairs", "bconv_cpt", "split_rows_alone",
+                                                                  "min_branch_pairs"]}
     c1 = Ciphertext(ctx, _random_pairs(ctx, pairs, 2))
     c2 = Ciphertext(ctx, _random_pairs(ctx, pairs, 3))
     out = Ciphertext(ctx, count=pairs)
@@ -220,9 +221,6 @@ def tune_pipeline(scheme, pairs: int = 64, reps: int = 5) -> Dict[str, object]:
     d1 = Ciphertext(ctx, c1.cipher_device[:two].clone())
     d2 = Ciphertext(ctx, c2.cipher_device[:two].clone())
     out2 = Ciphertext(ctx, count=two)
-    e1 = Ciphertext(ctx, c1.cipher_device[:1].clone())
-    e2 = Ciphertext(ctx, c2.cipher_device[:1].clone())
-    out1 = Ciphertext(ctx, count=1)
     eight = min(8, pairs)
     f1 = Ciphertext(ctx, c1.cipher_device[:eight].clone())
     f2 = Ciphertext(ctx, c2.cipher_device[:eight].clone())
@@ -236,16 +234,15 @@ def tune_pipeline(scheme, pairs: int = 64, reps: int = 5) -> Dict[str, object]:
         for k, vals in PIPELINE_KNOBS.items():  # defaults first: the reference products
             ctx.tune_set(k, vals[0])
         ctx.tune_set("k5_fused_pairs", K5_FUSED_PAIRS[0])
-        ctx.tune_set("fuse_q2r_pairs", FUSE_Q2R_PAIRS[0])
+        ctx.tune_set("bconv_cpt", BCONV_CPT[0])
         ctx.tune_set("split_rows_alone", SPLIT_ROWS_ALONE[0])
         ctx.tune_set("min_branch_pairs", MIN_BRANCH_PAIRS[0])
         scheme.mult_relin(c1, c2, out=out)
         scheme.mult_relin(d1, d2, out=out2)
-        scheme.mult_relin(e1, e2, out=out1)
         scheme.mult_relin(f1, f2, out=out8)
         scheme.mult_relin(g1, g2, out=out4)
         torch.cuda.synchronize()
-        want, want2, want1 = out.cipher_device.clone(), out2.cipher_device.clone(), out1.cipher_device.clone()
+        want, want2 = out.cipher_device.clone(), out2.cipher_device.clone()
         want8 = out8.cipher_device.clone()
         want4 = out4.cipher_device.clone()
         for k, vals in PIPELINE_KNOBS.items():
@@ -256,12 +253,13 @@ def tune_pipeline(scheme, pairs: int = 64, reps: int = 5) -> Dict[str, object]:
         result["k5_fused_pairs"], result["k5_fused_pairs_ms"] = min(ms, key=ms.get), {
             str(v): t for v, t in ms.items()}
 
-        def per_call():
-            scheme.mult_relin(e1, e2, out=out1)
-            scheme.mult_relin(d1, d2, out=out2)
-        ms = _sweep(ctx, "fuse_q2r_pairs", FUSE_Q2R_PAIRS, per_call, (out1, out2), (want1, want2), reps)
-        result["fuse_q2r_pairs"], result["fuse_q2r_pairs_ms"] = min(ms, key=ms.get), {
-            str(v): t for v, t in ms.items()}
+        result["fuse_q2r_pairs"], result["fuse_q2r_pairs_ms"] = ctx.tune_get("fuse_q2r_pairs"), {}
+        conv = Ciphertext(ctx, ctx.bconv_q_to_r(c1.cipher_device))
+
+        def convert():
+            conv.cipher_device = ctx.bconv_q_to_r(c1.cipher_device)
+        ms = _sweep(ctx, "bconv_cpt", BCONV_CPT, convert, conv, conv.cipher_device.clone(), reps)
+        result["bconv_cpt"], result["bconv_cpt_ms"] = min(ms, key=ms.get), {str(v): t for v, t in ms.items()}
 
         def small():
             scheme.mult_relin(g1, g2, out=out4)
@@ -284,7 +282,7 @@ def tune_pipeline(scheme, pairs: int = 64, reps: int = 5) -> Dict[str, object]:
 
 
 PIPELINE_CHOICES = ("branches", "bconv_threads", "bconv_cpt", "k5_threads", "split_rows", "l2_prefetch",
-                    "k5_fused_pairs", "fuse_q2r_pairs", "min_branch_pairs", "split_rows_alone")
+                    "k5_fused_pairs", "min_branch_pairs", "split_rows_alone")
 
 
 def apply_choice(ctx, choice: dict) -> None:
