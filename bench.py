@@ -562,9 +562,10 @@ def c4_uneven(stream):
 
 def step_roofline(ms_step, hbm_peak, peak_kind):
     """The headline step against its arithmetic bound: every primitive of the
-    pipeline counted per pair (kunpbfv_b200.roofline.pipeline_counts), those on the
-    IMAD pipe at the rates kbfv_probe_arith measures live on this GPU, the base
-    conversions' byte products at the tensor cores' (step_floor_s); and, from the
+    pipeline that the kernels issue, counted per pair
+    (kunpbfv_b200.roofline.pipeline_counts), those on the IMAD pipe at the rates
+    kbfv_probe_arith measures live on this GPU, the base conversions' byte
+    products at the tensor cores' (step_floor_s); and, from the
     committed ncu summary of the same kernel sources, the IMAD-pipe instructions
     per pair against the measured IMAD issue rate. Beside them the step's HBM
     rate (inputs, outputs and the key read once per launch)."""
@@ -577,11 +578,11 @@ def step_roofline(ms_step, hbm_peak, peak_kind):
     n = 1 << LOG_N
     bytes_pair = 4 * NQ * n * 8 + 2 * NQ * n * 8 + 2 * (NQ + NP) * n * 8 // BATCH
     out = {"bound": "imad", "unit": "modmul/s",
-           "modmuls_per_pair": pc["products"],
-           "reductions_per_pair": pc["counts"]["b128"],
-           "counts_per_pair": pc["counts"], "on_tensor_cores_per_pair": pc["conversions"], "ntt_rows_per_pair": pc["ntt_rows"], "formula": pc["formula"],
-           "achieved": round(pc["products"] * BATCH / step_s, 0),
-           "peak": round(pc["products"] / floor_s, 0),
+           "modmuls_per_pair": pc["issued_products"],
+           "counts_per_pair": pc["issued"], "byte_macs_per_pair": pc["byte_macs"],
+           "ntt_rows_per_pair": pc["ntt_rows"], "formula": pc["formula"],
+           "achieved": round(pc["issued_products"] * BATCH / step_s, 0),
+           "peak": round(pc["issued_products"] / floor_s, 0),
            "frac": round(floor_s * BATCH / step_s, 4),
            "floor_ms_per_step": round(floor_s * BATCH * 1e3, 4), "ms_per_step": round(ms_step, 4),
            "peak_source": "each class at its kbfv_probe_arith rate (register chains, no memory traffic): " +
