@@ -111,17 +111,17 @@ static inline int resident_ctas_at(const void* kernel, int threads, int smem, in
     return cache[i];
 }
 
-// Allows `kernel` up to `bytes` of dynamic shared memory (without it a launch may
-// take 48 KB). The permission belongs to the kernel in one CUDA context, so it is
-// asked for at each launch (53 ns) instead of remembered per process, where another
-// GPU's context would go without; and always for the same value, the kernel's
-// largest at any CTA size, so that threads with different CTA sizes do not lower it
-// for one another.
+// Allows `kernel` the dynamic shared memory of a launch of `bytes` (without it a launch
+// may take 48 KB). The permission belongs to the kernel in one CUDA context, so it is
+// asked for at each such launch (53 ns) instead of remembered per process, where
+// another GPU's context would go without; and always for the same value, the kernel's
+// largest at any CTA size (`most`), so that threads with different CTA sizes do not
+// lower it for one another.
 constexpr int kPlainSmem = 48 << 10;
 template <class K>
-static inline void allow_smem(K kernel, int bytes) {
+static inline void allow_smem(K kernel, int bytes, int most) {
     if (bytes > kPlainSmem)
-        KB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        KB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 }
 
 // A launch of clusters of `cluster` CTAs. `early`: it may start while the kernel
@@ -184,7 +184,7 @@ static void launch_inv_cluster(const DevConsts& dc, Src s, Dst d, int rows, cuda
 template <int LOGB, class Src, class Dst, bool FULL = true>
 static void launch_fwd_block(const DevConsts& dc, Src s, Dst d, int rows, int logn, cudaStream_t st) {
     constexpr int SMEM = BlockShape<LOGB>::SMEM_BYTES;
-    allow_smem(ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>, SMEM);
+    allow_smem(ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>, SMEM, SMEM);
     // CTAs of this kernel resident at once on the device
     static const int resident = resident_ctas((const void*)ntt_fwd_block_kernel<LOGB, Src, Dst, FULL>,
                                               BlockShape<LOGB>::THREADS, SMEM);
@@ -196,7 +196,7 @@ static void launch_fwd_block(const DevConsts& dc, Src s, Dst d, int rows, int lo
 template <int LOGB, class Src, class Dst, bool WHOLE>
 static void launch_inv_block(const DevConsts& dc, Src s, Dst d, int rows, int logn, cudaStream_t st) {
     constexpr int SMEM = BlockShape<LOGB>::SMEM_BYTES;
-    allow_smem(ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>, SMEM);
+    allow_smem(ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>, SMEM, SMEM);
     // CTAs of this kernel resident at once on the device
     static const int resident = resident_ctas((const void*)ntt_inv_block_kernel<LOGB, Src, Dst, WHOLE>,
                                               BlockShape<LOGB>::THREADS, SMEM);

@@ -251,7 +251,7 @@ static void ext_mma_launch_sh(const Job& job, int polys, int logn, int threads, 
                threads / 32 * 2 * 4 * KS * kRow<mma_tiles(KS)> * 8;
     };
     const int smem = smem_of(threads);
-    allow_smem(ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, smem_of(512));
+    allow_smem(ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, smem, smem_of(512));
     const int each = threads / 2 * mma_tiles(KS);
     const int iters = mma_iters(polys, logn, each,
                                 resident_ctas_at((const void*)ext_mma_kernel<KS, NG, EXTRA, PREP, SH, Job>, threads, smem, res));
@@ -594,7 +594,7 @@ static void k5_mma_launch_sh(const Job& job, int polys, int logn, int threads, c
     };
     const int smem = smem_of(threads);
     const int each = threads / 2 * mma_tiles(KS);
-    allow_smem(k5_mma_kernel<KS, NG, FUSED, SH, Job>, smem_of(256));
+    allow_smem(k5_mma_kernel<KS, NG, FUSED, SH, Job>, smem, smem_of(256));
     const int iters = mma_iters(polys, logn, each,
                                 resident_ctas_at((const void*)k5_mma_kernel<KS, NG, FUSED, SH, Job>, threads, smem, res));
     k5_mma_kernel<KS, NG, FUSED, SH, Job><<<mma_blocks(polys, logn, each, iters), threads, smem, st>>>(job, logn, iters);
