@@ -94,9 +94,12 @@ static __global__ void __launch_bounds__(256) lift_mma_kernel(Job job, int logn,
 template <int KS, class Job>
 static void lift_mma_launch(const Job& job, size_t table, int rows, int logn, int alpha, int threads, cudaStream_t st) {
     const int each = threads / 2 * mma_tiles(KS);
-    const int smem = table <= 16 << 10 ? (int)table : 0;  // larger tables are read through L1
-    const int iters =
-        mma_iters(rows, logn, each, resident_ctas((const void*)lift_mma_kernel<KS, Job>, threads, smem));
+    constexpr int kStaged = 16 << 10;  // larger tables are read through L1
+    const int smem = table <= kStaged ? (int)table : 0;
+    // resident CTAs with the largest staged table (registers bound them before that) and with none
+    static int res[2][4] = {};
+    const int iters = mma_iters(rows, logn, each, resident_ctas_at((const void*)lift_mma_kernel<KS, Job>, threads,
+                                                                    smem ? kStaged : 0, res[smem ? 1 : 0]));
     lift_mma_kernel<KS, Job><<<mma_blocks(rows, logn, each, iters), threads, smem, st>>>(job, logn, alpha, iters, smem != 0);
     check_launch("digit_lift");
 }
