@@ -111,9 +111,6 @@ __device__ __forceinline__ uint64_t barrett_prod_lazy(u128 x, uint64_t q, uint64
     const uint64_t t = (x.lo >> s) | (x.hi << (64 - s));
     return x.lo - __umul64hi(t, mu) * q;
 }
-__device__ __forceinline__ uint64_t mul_mod_prod(uint64_t a, uint64_t b, uint64_t q, uint64_t mu) {
-    return barrett_prod(mul_wide(a, b), q, mu);
-}
 
 // 64-bit value mod q with the high word of mu: floor(a * mu_hi / 2^64) errs by at most 1
 __device__ __forceinline__ uint64_t barrett64(uint64_t a, uint64_t q, uint64_t mu_hi) {

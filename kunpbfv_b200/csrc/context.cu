@@ -186,8 +186,6 @@ void build_context(Context& c, const kbfv_params& prm) {
     }
 
     DevConsts& dc = c.dc;
-    // two coefficients per base-conversion thread: 16% fewer IMAD instructions,
-    // 8% faster than one at N=16384, 7 + 1 primes, 32-pair sub-batches (B200)
     int sms = 0, dev = 0;
     KB_CHECK_CUDA(cudaGetDevice(&dev));
     KB_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -781,7 +779,8 @@ int kbfv_reserve(kbfv_context* ctx, uint32_t pairs) {
         std::lock_guard<std::mutex> lk(c.mu);
         const int chunk = (int)std::min<uint32_t>(std::max<uint32_t>(pairs, 1), kMaxBatch);
         size_t need = mul_scratch_need(c, chunk);
-        // encryption work area: 4 polys x nq per item; secret/relin keygen: 2*(nq+np)
+        // 4 polynomials over Q an item: more than encryption (v over Q, -Q m mod t and three
+        // byte polynomials) and the smaller calls take
         need = std::max(need, (size_t)chunk * 4 * c.nq * c.n * 8);
         ensure_scratch(c, need);
     });

@@ -147,7 +147,8 @@ static void launch_clusters(bool early, void (*kernel)(P...), unsigned grid, uns
 }
 
 // Whether a launch of `rows` rows runs on clusters (ntt_cluster.cuh): where that
-// takes less time than the other forms (148 SMs; us, cluster / other):
+// takes less time than the other forms. The limits are measured on 148 SMs and for
+// that chip only (us, cluster / other):
 //   2^12: 128 rows 9.3 / 10.4, 148 rows 13.1 / 10.4      2^13: 128 rows 15.2 / 16.6, 148 rows 17.8 / 16.6
 //   2^14: 8 rows 9.5 / 14.4, 26 rows 17 / 14.4 (the split form's single wave of up to
 //         148 quarter-row CTAs, against more than one cluster CTA per SM),
@@ -220,8 +221,9 @@ static inline Dst plain_of(const Dst& d) { return d; }
 constexpr int kSplitRows14Default = 48;
 // The same threshold for a multiply that runs as one stream (batches below two
 // sub-batches, the tensor-only multiply), where no sibling sub-batch fills the SMs
-// that few whole-ring CTAs leave idle. The
-// default of LaunchShape::split_rows_alone (KBFV_TUNE_SPLIT_ROWS_ALONE).
+// that few whole-ring CTAs leave idle. Clusters take up to 112 of these rows; from there
+// to 148 the split form is the slower one (33 us, whole rows 27), and a caller may set
+// fewer. The default of LaunchShape::split_rows_alone (KBFV_TUNE_SPLIT_ROWS_ALONE).
 constexpr int kSplitRowsAloneDefault = 148;
 
 // A wave of whole-ring CTAs of 2^14 points (one per SM) takes 25 us however few

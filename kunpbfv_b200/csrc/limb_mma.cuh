@@ -6,8 +6,9 @@
 //   sum_i w_i c_ij  =  sum_{i,b} w_{i,b} [2^(8b) c_ij mod m_j]   (mod m_j):
 // with the bytes of all words as the inner dimension and the eight base-256
 // digits of the constants as columns, one u8 matrix product gives, per output,
-// eight 24-bit digit sums whose weighted sum is below 2^77 (60-bit constants,
-// at most 36 words), and one 17-bit quotient reduces it. Against 64-bit
+// eight 24-bit digit sums whose weighted sum is below 2^77 (60-bit constants;
+// at most 35 words below 2^60 and a rounding quotient of any 64 bits), and one 17-bit
+// quotient reduces it. Against 64-bit
 // multiply-accumulates into 128 bits and a 128-bit Barrett reduction that is
 // about a third of the multiply-pipe work of a conversion (8 MACs of eight
 // 32-bit products each and four high products per output become one wide, one
@@ -101,7 +102,8 @@ __device__ __forceinline__ void imma(int (&c)[4], uint32_t a0, uint32_t a1, uint
 // Digit sums of output group G for MT tiles of 16 coefficients: D[m][h][2 * row
 // + e] is digit 2h + 256 * digit 2h + 1 of output (G, e) of the lane's
 // coefficient `row` of tile m. A pair of digit tiles is combined as soon as it is
-// summed (the digit sums stay below 2^24, so the pair fits 32 bits), which keeps
+// summed (35 words below 2^60, their top byte below 16, and one full word
+// keep the digit sums below 2^24, so the pair fits 32 bits), which keeps
 // 16 instead of 32 registers of sums per tile, and one load of the constants
 // (tab: in shared memory) serves MT tiles.
 template <int KS, int MT>

@@ -595,7 +595,9 @@ void ks_tail(const DevConsts& dc, const uint64_t* sd2, const uint64_t* key, int 
              const uint64_t* add, const PtrBatch& pb, int count, cudaStream_t st, const KsExtra& ex = {});
 // the auxiliary streams and fork / join events of the sub-batches (created once)
 void ensure_branch_streams(Context& c);
-// the whole multiply + relinearise of one sub-batch (9 launches)
+// the whole multiply + relinearise of one sub-batch: K1..K5, the lift, K6a, K6b and K7
+// (one launch less where the lift is inside K5 or K6a, one more for key products
+// apart, and for each transform that takes two)
 void mul_relin_chunk(const DevConsts& dc, const uint64_t* rlk, const PtrBatch& pb, int count, const MulScratch& m,
                      cudaStream_t st);
 // the constants of a sub-batch beside another on a sibling stream

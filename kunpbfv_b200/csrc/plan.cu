@@ -1,6 +1,6 @@
 // Captured multiplies (kbfv_plan_*): a caller that multiplies the same device
 // buffers again and again (a request loop with fixed staging buffers) replays
-// the whole multiply as one CUDA graph launch instead of issuing its 8 to 12
+// the whole multiply as one CUDA graph launch instead of issuing its 8 to 15
 // kernel launches one by one; a batch of pairs at mixed levels
 // (kbfv_mul_relin_levels) likewise becomes one graph launch. No counterpart in
 // the reference.
@@ -47,8 +47,8 @@ bool graph_current(const kbfv_plan& p) {
            std::memcmp(&c.dc.shape, &p.shape, sizeof(LaunchShape)) == 0;
 }
 
-// Runs the multiply on `st` (eagerly: first-use set-up such as module loading,
-// kernel attributes and scratch growth happens here, outside any capture),
+// Runs the multiply on `st` (eagerly: first-use set-up such as module loading and
+// scratch growth happens here, outside any capture),
 // then records the same launch sequence on the plan's own stream into a graph.
 // Capturing executes nothing.
 int run_once(kbfv_plan& p, cudaStream_t st) {
