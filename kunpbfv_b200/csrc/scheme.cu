@@ -246,6 +246,10 @@ struct AddPlainDst {  // rows (item, l) of the b parts
         return AddPlainRow{ct + at, out + at, dc.mods[l]};
     }
 };
+// whether two ranges of words share one
+static inline bool overlap(const uint64_t* a, size_t na, const uint64_t* b, size_t nb) {
+    return (uintptr_t)a < (uintptr_t)(b + nb) && (uintptr_t)b < (uintptr_t)(a + na);
+}
 static inline RowsIO plain_of(const AddPlainDst& d) { return RowsIO{d.rows, d.dc.logn, 0, d.dc.nq}; }
 
 // x = pb.a[item], y = pb.b[item], out = pb.o[item]: 2 x nq limbs each; grid.y = item
@@ -510,11 +514,28 @@ int kbfv_add_plain(kbfv_context* ctx, const uint64_t* d_ct, const uint64_t* d_m,
             const int cnt = (int)std::min<uint32_t>(kMaxBatch, count - off);
             const uint64_t* src = d_ct + (size_t)off * 2 * lq;
             uint64_t* dst = d_out + (size_t)off * 2 * lq;
-            uint64_t* rows = (uint64_t*)ensure_scratch(c, (size_t)cnt * lq * 8);
-            ntt_fwd(c.dc, DeltaSrc{d_m + (size_t)off * c.n, c.dc}, AddPlainDst{src, dst, rows, c.dc}, cnt * c.nq, st);
-            if (dst != src)  // the a parts
-                KB_CHECK_CUDA(cudaMemcpy2DAsync(dst, 2 * lq * 8, src, 2 * lq * 8, lq * 8, (size_t)cnt,
-                                                cudaMemcpyDeviceToDevice, st));
+            const uint64_t* m = d_m + (size_t)off * c.n;
+            // The transform of all items reads and writes at once. Plaintexts that lie in the
+            // output are copied aside first; an output shifted against its input is written
+            // item by item, a part first, so that no item is overwritten before it is read.
+            const bool m_in_out = overlap(m, cnt * c.n, dst, cnt * 2 * lq);
+            const bool shifted = dst != src && overlap(src, cnt * 2 * lq, dst, cnt * 2 * lq);
+            uint64_t* rows = (uint64_t*)ensure_scratch(c, (size_t)cnt * (lq + (m_in_out ? c.n : 0)) * 8);
+            if (m_in_out) {
+                KB_CHECK_CUDA(cudaMemcpyAsync(rows + cnt * lq, m, (size_t)cnt * c.n * 8, cudaMemcpyDeviceToDevice, st));
+                m = rows + cnt * lq;
+            }
+            auto copy_a = [&](size_t i, int items) {
+                KB_CHECK_CUDA(cudaMemcpy2DAsync(dst + i * 2 * lq, 2 * lq * 8, src + i * 2 * lq, 2 * lq * 8, lq * 8,
+                                                (size_t)items, cudaMemcpyDeviceToDevice, st));
+            };
+            const int step = shifted ? 1 : cnt;
+            for (size_t i = 0; i < (size_t)cnt; i += step) {
+                if (shifted) copy_a(i, 1);
+                ntt_fwd(c.dc, DeltaSrc{m + i * c.n, c.dc}, AddPlainDst{src + i * 2 * lq, dst + i * 2 * lq, rows, c.dc},
+                        step * c.nq, st);
+            }
+            if (dst != src && !shifted) copy_a(0, cnt);
         }
     });
 }
