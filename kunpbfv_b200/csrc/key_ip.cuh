@@ -83,7 +83,17 @@ static __global__ void __launch_bounds__(256, C * O > 8 ? 2 : 3) key_ip_kernel(K
 }
 
 template <int O>
-static void key_ip_launch(const DevConsts& dc, const KeyIpJob& J, cudaStream_t st) {
+static void key_ip_launch(const DevConsts& dc, KeyIpJob J, cudaStream_t st) {
+    // a launch takes up to 65535 groups of four items
+    constexpr int kItems = 65535 * 4;
+    for (; J.items > kItems; J.items -= kItems) {
+        KeyIpJob part = J;
+        part.items = kItems;
+        key_ip_launch<O>(dc, part, st);
+        J.dig += kItems * J.dig_item;
+        J.out += kItems * J.out_item;
+        if (J.extra) J.extra += kItems * J.extra_item;
+    }
     if (J.items <= 0) return;
     const int groups = (J.items + 3) / 4, per = (J.items + groups - 1) / groups;
     const dim3 grid((1u << dc.logn) / 256, (unsigned)(J.limbs * ((J.outputs + O - 1) / O)),
